@@ -141,7 +141,7 @@ __host__ __device__ inline int staged_doubles(int32_t kind) {
 
 /*
  * Shared-memory image of one cell for a window (all sizes in elements):
- *   doubles  v, d, rhs, a [n each]; eliminated pivot and rhs contributions of
+ *   doubles  d and rhs [n + 2 pairs], a [n + 2], v [n]; eliminated pivot and rhs contributions of
  *            chain tops [nch each]; event increments [inbox_cap]; staged FP64
  *            slots of the staged rows;
  *   events   the cell's inbox for the window [inbox_cap];
@@ -158,7 +158,7 @@ struct CellShape {
 
 __host__ __device__ inline size_t cell_smem_bytes(const CellShape &s, const int32_t *kinds, int32_t ngroups,
                                                   int32_t inbox_cap) {
-    size_t doubles = 4 * (size_t)s.n + 2 * (size_t)s.nch + (size_t)inbox_cap;
+    size_t doubles = 4 * (size_t)s.n + 6 + 2 * (size_t)s.nch + (size_t)inbox_cap;
     size_t ints = 0;
     for (int32_t g = 0; g < ngroups; ++g) {
         if (!kind_staged(kinds[g])) continue;
@@ -196,6 +196,7 @@ struct Params {
     const int32_t *path_off;     // [ncells+1] into path_chain
     const int32_t *path_chain;   // per cell: npaths+1 local chain starts; only the sentinel for a
                                  // cell on the chain schedule (its paths are its chains)
+    int32_t axial_ok;          // every axial conductance is 0 or in [2^-480, 2^480)
     DevGroup groups[kMaxGroups];
     // per cell, group and thread: first row (relative to the cell's first row of the group)
     // of the thread's rows; thread t owns the local nodes i with i % kCellThreads == t

@@ -485,210 +485,165 @@ __device__ __forceinline__ void apply_event(const StagedGroup &G, int32_t row, d
     }
 }
 
+__device__ __forceinline__ bool bad_pivot(double D) { return (D == 0.0) | !isfinite(D); }
+
+/* Where the quotients below are exact: magnitudes in [2^-480, 2^480), where nothing can overflow
+ * or lose bits to underflow, and for the divisor no significand that starts with twenty ones (of
+ * which the all-ones one is an exception of the method).  A quotient in [2^-400, 2^400) of a
+ * divisor in range came from a numerator in range, and a zero from a zero or from an underflow
+ * that the division shares. */
+__device__ __forceinline__ bool in_binades(double x, uint32_t low, uint32_t high) {
+    return ((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) - (low << 20) < (high - low) << 20;
+}
+__device__ __forceinline__ bool good_divisor(double D) {
+    return in_binades(D, 1023u - 480u, 1023u + 480u) && (((uint32_t)__double2hiint(D) + 1u) & 0xFFFFFu) != 0u;
+}
+__device__ __forceinline__ bool good_quotient(double x) { return x == 0.0 || in_binades(x, 1023u - 400u, 1023u + 400u); }
+
 /*
- * Hines solve of one resident cell, FP64 mode: the reference's operations in the
- * canonical order (gather-form elimination, f = a/D, back-substitution (R + a x_p)/D).
- * Level by level, one path per thread (a path is one chain, or a chain and the child chains
- * it continues when the cell's plan merged them): a path's chains are eliminated deepest
- * first and back-substituted in the reverse order, each child chain ready before its parent
- * (on the path, by the same thread; off it, in a lower level).  Along a chain only subtract
- * -> divide -> multiply stays on the dependency chain, the next node's operands being
- * loaded before the current division.  pch null: the cell's paths are its chains (lvp holds
- * chain starts), the loops are the one-chain-per-thread loops.
+ * IEEE quotients of the FP64 solve without the division's branches (a dependent division
+ * measured 127 cycles on a B200, an FP64 fma 8.6, rcp.approx.ftz.f64 17.7), after
+ * P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
+ * processor", IBM J. Res. Dev. 34(1), 1990, and J.-M. Muller et al., Handbook of
+ * Floating-Point Arithmetic, chapter on FMA-based division:
+ *   - two Newton steps on a seed good to 2^-19 leave y2 within one unit in the last place of
+ *     1/D, and a third, y3 = y2 + y2 (1 - D y2) with the residual exact in one FMA, rounds to
+ *     the nearest double of 1/D;
+ *   - q1 = q0 + (n - D q0) y is within one unit in the last place of n/D, its residual
+ *     r1 = n - D q1 is exact, and q1 + r1 y3 rounds to the IEEE quotient.
  */
-template <int NT>
-__device__ __forceinline__ void hines_exact(double *sd, double *sr, const double *sa, double *sv, double *sxd,
-                                            double *sxr, const int32_t *ctop, const int32_t *clen,
-                                            const int32_t *cpar, const int32_t *ckoff, const int32_t *ckids,
-                                            const int32_t *lvp, const int32_t *pch, int32_t nlev, double vscale,
-                                            bool &singular) {
-    constexpr int32_t T = NT;
-    const int32_t tid = threadIdx.x;
-    for (int32_t lv = 0; lv < nlev; ++lv) {
-        for (int32_t p = lvp[lv] + tid; p < lvp[lv + 1]; p += T)
-        for (int32_t ch = pch ? pch[p] : p, end = pch ? pch[p + 1] : p + 1; ch < end; ++ch) {
-            const int32_t top = ctop[ch];
-            const int32_t bottom = top + clen[ch] - 1;
-            const bool rooted = cpar[ch] < 0;
-            double D = sd[bottom], R = sr[bottom];
-            for (int32_t q = ckoff[ch]; q < ckoff[ch + 1]; ++q) {
-                const int32_t cc = ckids[q];
-                D = D - sxd[cc];
-                R = R + sxr[cc];
-            }
-            singular |= (D == 0.0) | !isfinite(D);
-            sd[bottom] = D;
-            sr[bottom] = R;
-            double pxd = 0.0, pxr = 0.0;
-            if (bottom > top || !rooted) {
-                const double ab = sa[bottom];
-                double dn = 0.0, rn = 0.0, an = 0.0;
-                if (bottom > top) {
-                    dn = sd[bottom - 1];
-                    rn = sr[bottom - 1];
-                    an = sa[bottom - 1];
-                }
-                const double f = ab / D;
-                pxd = f * ab;
-                pxr = f * R;
-                // interior nodes: every one has its parent at i - 1
-                int32_t i = bottom - 1;
-                for (; i > top; --i) {
-                    const double Di = dn - pxd, Ri = rn + pxr, ai = an;
-                    dn = sd[i - 1];
-                    rn = sr[i - 1];
-                    an = sa[i - 1];
-                    singular |= (Di == 0.0) | !isfinite(Di);
-                    sd[i] = Di;
-                    sr[i] = Ri;
-                    const double fi = ai / Di;
-                    pxd = fi * ai;
-                    pxr = fi * Ri;
-                }
-                if (i == top && bottom > top) {
-                    const double Dt = dn - pxd, Rt = rn + pxr;
-                    singular |= (Dt == 0.0) | !isfinite(Dt);
-                    sd[top] = Dt;
-                    sr[top] = Rt;
-                    if (!rooted) {
-                        const double ft = an / Dt;
-                        pxd = ft * an;
-                        pxr = ft * Rt;
-                    }
-                }
-            }
-            sxd[ch] = pxd;
-            sxr[ch] = pxr;
-        }
-        __syncthreads();
-    }
-    for (int32_t lv = nlev - 1; lv >= 0; --lv) {
-        for (int32_t p = lvp[lv] + tid; p < lvp[lv + 1]; p += T)
-        for (int32_t ch = (pch ? pch[p + 1] : p + 1) - 1, first = pch ? pch[p] : p; ch >= first; --ch) {
-            const int32_t top = ctop[ch];
-            const int32_t bottom = top + clen[ch] - 1;
-            const int32_t par = cpar[ch];
-            double rn = sr[top], an = sa[top], dn = sd[top];
-            double x;
-            {
-                const double ri = rn, ai = an, di = dn;
-                const double xp = par >= 0 ? sr[par] : 0.0;
-                if (top < bottom) {
-                    rn = sr[top + 1];
-                    an = sa[top + 1];
-                    dn = sd[top + 1];
-                }
-                x = (par >= 0 ? ri + ai * xp : ri) / di;
-                sr[top] = x;
-                sv[top] = sv[top] + vscale * x;
-            }
-            for (int32_t i = top + 1; i <= bottom; ++i) {
-                const double ri = rn, ai = an, di = dn;
-                if (i < bottom) {
-                    rn = sr[i + 1];
-                    an = sa[i + 1];
-                    dn = sd[i + 1];
-                }
-                x = (ri + ai * x) / di;
-                sr[i] = x;
-                sv[i] = sv[i] + vscale * x;
-            }
-        }
-        __syncthreads();
-    }
+__device__ __forceinline__ double reciprocal_seed(double D) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(D));
+    return y;
+}
+__device__ __forceinline__ double reciprocal(double D) {
+    double y = reciprocal_seed(D);
+    y = fma(y, fma(-D, y, 1.0), y);
+    y = fma(y, fma(-D, y, 1.0), y);
+    return fma(y, fma(-D, y, 1.0), y);
+}
+/* n / D from D's reciprocal. */
+__device__ __forceinline__ double quotient(double n, double D, double y) {
+    const double q0 = n * y;
+    const double q1 = fma(fma(-D, q0, n), y, q0);
+    return fma(fma(-D, q1, n), y, q1);
+}
+/* a / D with D just known: the quotient starts from the reciprocal's first iterate. */
+__device__ __forceinline__ double pivot_quotient(double a, double D) {
+    const double y0 = reciprocal_seed(D);
+    const double y1 = fma(y0, fma(-D, y0, 1.0), y0);
+    const double q0 = a * y1;
+    const double y2 = fma(y1, fma(-D, y1, 1.0), y1);
+    const double q1 = fma(fma(-D, q0, a), y2, q0);
+    const double y3 = fma(y2, fma(-D, y2, 1.0), y2);
+    return fma(fma(-D, q1, a), y3, q1);
 }
 
 /*
- * Hines solve, mixed mode: FP64 arithmetic with reciprocals.  Elimination keeps, per
- * node, f = a/D in place of D and R/D in place of R, so the back-substitution is one
- * FMA per node, x = f x_p + R/D; the pivot chain is D -> 1/D -> (a^2)(1/D) -> next D.
- * One path per thread, level by level, as in the FP64 solve.
+ * Hines solve of one resident cell, level by level, one path per thread: a path is one chain, or a
+ * chain and the child chains it continues when the cell's plan merged them; a path's chains
+ * are eliminated deepest first and back-substituted in the reverse order, each child chain ready
+ * before its parent (on the path, by the same thread; off it, in a lower level).  pch null: the
+ * cell's paths are its chains (lvp holds chain starts), the loops are the one-chain-per-thread
+ * loops.  The solution is left in sdr[].y.
+ *
+ * FP64 mode: the reference's operations in the canonical order (gather-form elimination, f = a/D,
+ * back-substitution (R + a x_p)/D), the quotients by pivot_quotient and quotient; the caller
+ * checks afterwards that every one was in their range, and repeats the solve with EXACT,
+ * which divides, where one was not.  Mixed mode: f = a y and R y in place of D and R with
+ * y = approx_reciprocal(D), so the back-substitution is one FMA per node, x = f x_p + R y.
+ *
+ * What bounds it is the instructions of a node: the few lanes that hold the level's longest
+ * chains issue one every 4 to 5 cycles (measured).  So the sweeps hold the recurrence and its
+ * loads and stores only, the next node's operands loaded a node ahead (sdr and sa have a guard
+ * element at either end for it); the range checks and the voltage update are the caller's, on
+ * all threads.  Measured against divisions, pivot tests and updates inside the sweeps (window
+ * kernel, us per step): 64 ball-and-stick cells 14.2 -> 11.7, 4,000 random trees 249 -> 195,
+ * 250 pyramidal cells 98 -> 81 (FP64); 1,500 random trees 59 -> 54, 1,000 pyramidal cells
+ * 79 -> 73 (mixed).
  */
-template <int NT>
-__device__ __forceinline__ void hines_mixed(double *sd, double *sr, const double *sa, double *sv, double *sxd,
-                                            double *sxr, const int32_t *ctop, const int32_t *clen,
-                                            const int32_t *cpar, const int32_t *ckoff, const int32_t *ckids,
-                                            const int32_t *lvp, const int32_t *pch, int32_t nlev, double vscale,
-                                            bool &singular) {
+template <bool MIXED, bool EXACT, int NT>
+__device__ __forceinline__ void hines(double2 *sdr, const double *sa, double *sxd, double *sxr, const int32_t *ctop,
+                                      const int32_t *clen, const int32_t *cpar, const int32_t *ckoff,
+                                      const int32_t *ckids, const int32_t *lvp, const int32_t *pch, int32_t nlev,
+                                      bool &singular) {
     constexpr int32_t T = NT;
     const int32_t tid = threadIdx.x;
     for (int32_t lv = 0; lv < nlev; ++lv) {
         for (int32_t p = lvp[lv] + tid; p < lvp[lv + 1]; p += T)
         for (int32_t ch = pch ? pch[p] : p, end = pch ? pch[p + 1] : p + 1; ch < end; ++ch) {
-            const int32_t top = ctop[ch];
-            const int32_t bottom = top + clen[ch] - 1;
-            const bool rooted = cpar[ch] < 0;
-            double D = sd[bottom], R = sr[bottom];
+            const int32_t nodes = clen[ch];
+            const int32_t bottom = ctop[ch] + nodes - 1;
+            double2 *at = sdr + bottom;
+            const double *pa = sa + bottom;
+            double2 dr = *at;
+            double a = *pa;
             for (int32_t q = ckoff[ch]; q < ckoff[ch + 1]; ++q) {
                 const int32_t cc = ckids[q];
-                D = D - sxd[cc];
-                R = R + sxr[cc];
+                dr.x = dr.x - sxd[cc];
+                dr.y = dr.y + sxr[cc];
             }
-            singular |= (D == 0.0) | !isfinite(D);
-            const double ab = sa[bottom];
-            double dn = 0.0, rn = 0.0, an = 0.0;
-            if (bottom > top) {
-                dn = sd[bottom - 1];
-                rn = sr[bottom - 1];
-                an = sa[bottom - 1];
+            double xd = 0.0, xr = -0.0;   // neutral: nothing below the bottom on this chain
+#pragma unroll 2
+            for (int32_t k = 0; k < nodes; ++k) {
+                const double D = dr.x - xd, R = dr.y + xr, ai = a;
+                dr = at[-1];
+                a = pa[-1];
+                double f;
+                if (MIXED) {
+                    const double y = approx_reciprocal(D);
+                    f = ai * y;
+                    *at = make_double2(f, R * y);
+                    xd = (ai * ai) * y;
+                } else {
+                    *at = make_double2(D, R);
+                    if (EXACT) {
+                        singular |= bad_pivot(D);
+                        f = ai / D;
+                    } else {
+                        f = pivot_quotient(ai, D);
+                    }
+                    xd = f * ai;
+                }
+                xr = f * R;
+                --at;
+                --pa;
             }
-            const double y = approx_reciprocal(D);
-            const double f = ab * y;
-            sd[bottom] = f;
-            sr[bottom] = R * y;
-            double pxd = (ab * ab) * y, pxr = f * R;
-            int32_t i = bottom - 1;
-            for (; i > top; --i) {
-                const double Di = dn - pxd, Ri = rn + pxr, ai = an, asq = an * an;
-                dn = sd[i - 1];
-                rn = sr[i - 1];
-                an = sa[i - 1];
-                singular |= (Di == 0.0) | !isfinite(Di);
-                const double yi = approx_reciprocal(Di);
-                const double fi = ai * yi;
-                sd[i] = fi;
-                sr[i] = Ri * yi;
-                pxd = asq * yi;
-                pxr = fi * Ri;
-            }
-            if (bottom > top) {
-                const double Dt = dn - pxd, Rt = rn + pxr;
-                singular |= (Dt == 0.0) | !isfinite(Dt);
-                const double yt = approx_reciprocal(Dt);
-                const double ft = an * yt;
-                sd[top] = ft;
-                sr[top] = Rt * yt;
-                pxd = (an * an) * yt;
-                pxr = ft * Rt;
-            }
-            sxd[ch] = rooted ? 0.0 : pxd;
-            sxr[ch] = rooted ? 0.0 : pxr;
+            sxd[ch] = xd;
+            sxr[ch] = xr;
         }
         __syncthreads();
     }
     for (int32_t lv = nlev - 1; lv >= 0; --lv) {
         for (int32_t p = lvp[lv] + tid; p < lvp[lv + 1]; p += T)
         for (int32_t ch = (pch ? pch[p + 1] : p + 1) - 1, first = pch ? pch[p] : p; ch >= first; --ch) {
-            const int32_t top = ctop[ch];
-            const int32_t bottom = top + clen[ch] - 1;
-            const int32_t par = cpar[ch];
-            double fn = sd[top], qn = sr[top];
-            double x = par >= 0 ? fma(fn, sr[par], qn) : qn;
-            sr[top] = x;
-            sv[top] = sv[top] + vscale * x;
-            if (top < bottom) {
-                fn = sd[top + 1];
-                qn = sr[top + 1];
-            }
-            for (int32_t i = top + 1; i <= bottom; ++i) {
-                const double fi = fn, qi = qn;
-                if (i < bottom) {
-                    fn = sd[i + 1];
-                    qn = sr[i + 1];
+            const int32_t nodes = clen[ch], par = cpar[ch];
+            double2 *at = sdr + ctop[ch];
+            const double *pa = sa + ctop[ch];
+            double2 dr = *at;
+            double a = MIXED ? 0.0 : *pa;
+            double x = par >= 0 ? sdr[par].y : -0.0;   // a root's missing parent adds nothing
+            double y = MIXED || EXACT ? 1.0 : reciprocal(dr.x);
+#pragma unroll 2
+            for (int32_t k = 0; k < nodes; ++k) {
+                const double D = dr.x, R = dr.y, ai = a;
+                dr = at[1];
+                if (MIXED) {
+                    x = fma(D, x, R);
+                } else {
+                    a = pa[1];
+                    const double rhs = R + ai * x;
+                    if (EXACT) {
+                        x = rhs / D;
+                    } else {
+                        x = quotient(rhs, D, y);
+                        y = reciprocal(dr.x);
+                    }
+                    ++pa;
                 }
-                x = fma(fi, x, qi);
-                sr[i] = x;
-                sv[i] = sv[i] + vscale * x;
+                at->y = x;
+                ++at;
             }
         }
         __syncthreads();
@@ -734,10 +689,10 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     unsigned char *image = smem_raw;
     if (GLOBAL_IMAGE) image = P.big_image + (int64_t)P.big_slot[c] * P.big_stride;
     double *dp = reinterpret_cast<double *>(image);
+    // d and rhs, and a, with a guard element at either end
+    double2 *sdr = reinterpret_cast<double2 *>(dp) + 1; dp += 2 * (n + 2);
+    double *sa = dp + 1; dp += n + 2;
     double *sv = dp; dp += n;
-    double *sd = dp; dp += n;
-    double *sr = dp; dp += n;
-    double *sa = dp; dp += n;
     double *sxd = dp; dp += nch;
     double *sxr = dp; dp += nch;
     double *sw = dp; dp += P.inbox_cap;
@@ -892,6 +847,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     const float q10f = (float)q10;
     int32_t cursor = 0;
     bool singular = false;
+    bool exact = false;   // solve this step with divisions
 
     for (int32_t s = 0; s < W; ++s) {
         const int64_t step = n0 + s;
@@ -953,6 +909,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
             }
         }
         __syncthreads();  // NET_RECEIVE above wrote staged synapse state
+    assemble:
 
         // 3-5. Node i belongs to owner slot i % O and thread t serves the slots t, t + T, ...
         //      (a warp's lanes touch consecutive nodes, so shared memory serves them without
@@ -962,8 +919,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
         //      follows without a barrier (it reads only the unchanged v of neighbours).
         //      Parameters are streamed from HBM through the read-only path.
         for (int32_t i = tid; i < n; i += T) {
-            sd[i] = 0.0;
-            sr[i] = 0.0;
+            sdr[i] = make_double2(0.0, 0.0);
         }
         const double tc = t + 0.5 * P.dt;
         for (int32_t g = 0; g < P.ngroups; ++g) {
@@ -983,8 +939,8 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                         const double probe = vv + 0.001;
                         const double shifted = 0.0 + gp * (probe - ep);
                         const double value = 0.0 + gp * (vv - ep);
-                        sr[node] = sr[node] - scale * value;
-                        sd[node] = sd[node] + milli_quotient<MIXED>(scale * (shifted - value));
+                        sdr[node].y = sdr[node].y - scale * value;
+                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(scale * (shifted - value));
                     }
                 } else if (G.kind == MIND_MECH_ICLAMP) {
                     const int32_t *pn = GG.node + G.r0;
@@ -995,8 +951,8 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                         const double i = (tc < del + __ldg(GG.f[IC_DUR] + q) && tc >= del) ? __ldg(GG.f[IC_AMP] + q) : 0.0;
                         const double shifted = 0.0 - i;
                         const double value = 0.0 - i;
-                        sr[node] = sr[node] + -1.0 * value;
-                        sd[node] = sd[node] + milli_quotient<MIXED>(1.0 * (shifted - value));
+                        sdr[node].y = sdr[node].y + -1.0 * value;
+                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(1.0 * (shifted - value));
                     }
                 } else if (G.kind == MIND_MECH_ALPHASYN) {
                     // g = gmax alpha((t - onset)/tau), i = g (v - e) at the step's mid time
@@ -1009,15 +965,15 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                         const double e = __ldg(GG.f[AS_E] + q);
                         const double vv = sv[node];
                         if (MIXED) {  // linear in v: the probe's difference quotient is g
-                            sr[node] = sr[node] - gs * (vv - e);
-                            sd[node] = sd[node] + gs;
+                            sdr[node].y = sdr[node].y - gs * (vv - e);
+                            sdr[node].x = sdr[node].x + gs;
                             continue;
                         }
                         const double probe = vv + 0.001;
                         const double shifted = 0.0 + gs * (probe - e);
                         const double value = 0.0 + gs * (vv - e);
-                        sr[node] = sr[node] + -1.0 * value;
-                        sd[node] = sd[node] + milli_quotient<MIXED>(1.0 * (shifted - value));
+                        sdr[node].y = sdr[node].y + -1.0 * value;
+                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(1.0 * (shifted - value));
                     }
                 } else if (GEN && GG.gen >= 0) {
                     // emitted from a MOD file: BREAKPOINT probed at v + 0.001 and at v
@@ -1032,8 +988,8 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                         row.v = vv;
                         const double value = gen_current(GG.gen, row);
                         const double scale = pscale[r];
-                        sr[node] = sr[node] - scale * value;
-                        sd[node] = sd[node] + milli_quotient<MIXED>(scale * (shifted - value));
+                        sdr[node].y = sdr[node].y - scale * value;
+                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(scale * (shifted - value));
                     }
                 } else if (G.kind == MIND_MECH_HH) {
                     for (int32_t r = lo; r < hi; ++r) {
@@ -1049,8 +1005,8 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                             const double i = gl * (vv - G.at(HH_EL, r)) + gna * (vv - G.at(HH_ENA, r)) +
                                              gk * (vv - G.at(HH_EK, r));
                             const double scale = G.at(HH_SCALE, r);
-                            sr[node] = sr[node] - scale * i;
-                            sd[node] = sd[node] + scale * (gna + gk + gl);
+                            sdr[node].y = sdr[node].y - scale * i;
+                            sdr[node].x = sdr[node].x + scale * (gna + gk + gl);
                             continue;
                         }
                         const double shifted = hh_current(probe, m, h, nn, G.at(HH_GNABAR, r), G.at(HH_GKBAR, r),
@@ -1058,8 +1014,8 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                         const double value = hh_current(vv, m, h, nn, G.at(HH_GNABAR, r), G.at(HH_GKBAR, r),
                                                         G.at(HH_GL, r), G.at(HH_EL, r), G.at(HH_ENA, r), G.at(HH_EK, r));
                         const double scale = G.at(HH_SCALE, r);
-                        sr[node] = sr[node] - scale * value;
-                        sd[node] = sd[node] + milli_quotient<MIXED>(scale * (shifted - value));
+                        sdr[node].y = sdr[node].y - scale * value;
+                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(scale * (shifted - value));
                     }
                 } else if (G.kind == MIND_MECH_EXPSYN || G.kind == MIND_MECH_EXP2SYN) {
                     const bool two = G.kind == MIND_MECH_EXP2SYN;
@@ -1074,15 +1030,15 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                             gs = G.at(0, r);
                         const double vv = sv[node];
                         if (MIXED) {  // linear in v: the probe's difference quotient is the conductance
-                            sr[node] = sr[node] - gs * (vv - e);
-                            sd[node] = sd[node] + gs;
+                            sdr[node].y = sdr[node].y - gs * (vv - e);
+                            sdr[node].x = sdr[node].x + gs;
                             continue;
                         }
                         const double probe = vv + 0.001;
                         const double shifted = 0.0 + gs * (probe - e);
                         const double value = 0.0 + gs * (vv - e);
-                        sr[node] = sr[node] + -1.0 * value;
-                        sd[node] = sd[node] + milli_quotient<MIXED>(1.0 * (shifted - value));
+                        sdr[node].y = sdr[node].y + -1.0 * value;
+                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(1.0 * (shifted - value));
                     }
                 }
             }
@@ -1094,12 +1050,12 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
             const int32_t top = ctop[k];
             const int32_t bottom = top + clen[k] - 1;
             const double vi = sv[i];
-            double R = sr[i];
+            double R = sdr[i].y;
             if (MIXED) {
-                sd[i] = __ldg(P.mix_dc + gi) + sd[i];
+                sdr[i].x = __ldg(P.mix_dc + gi) + sdr[i].x;
                 R = R + (__ldg(P.mix_gse + gi) - __ldg(P.mix_gs + gi) * vi);
             } else {
-                sd[i] = (__ldg(P.cdt + gi) + sd[i]) + __ldg(P.ad + gi);
+                sdr[i].x = (__ldg(P.cdt + gi) + sdr[i].x) + __ldg(P.ad + gi);
             }
             const int32_t p = i == top ? cpar[k] : i - 1;
             if (p >= 0) R = R + sa[i] * (sv[p] - vi);
@@ -1111,19 +1067,34 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     R = R - sa[kt] * (vi - sv[kt]);
                 }
             }
-            sr[i] = R;
+            sdr[i].y = R;
         }
         __syncthreads();
 
-        // 6-7. Hines elimination level by level, each chain bottom to top into its parent,
-        //      then back-substitution root chain first with the voltage update.
+        // 6-7. Hines elimination level by level, each chain bottom to top into its parent, then
+        //      back-substitution root chain first, and the voltage update.
+        const int32_t *paths = PATHS && npath ? pch : nullptr;
+        if (exact)
+            hines<MIXED, true, NT>(sdr, sa, sxd, sxr, ctop, clen, cpar, ckoff, ckids, lvp, paths, nlev, singular);
+        else
+            hines<MIXED, false, NT>(sdr, sa, sxd, sxr, ctop, clen, cpar, ckoff, ckids, lvp, paths, nlev, singular);
         if (MIXED) {
-            hines_mixed<NT>(sd, sr, sa, sv, sxd, sxr, ctop, clen, cpar, ckoff, ckids, lvp,
-                          PATHS && npath ? pch : nullptr, nlev, P.vscale, singular);
+            for (int32_t i = tid; i < n; i += T) {
+                const double2 fx = sdr[i];
+                singular |= !isfinite(fx.x);   // a zero or non-finite pivot
+                sv[i] = sv[i] + P.vscale * fx.y;
+            }
         } else {
-            hines_exact<NT>(sd, sr, sa, sv, sxd, sxr, ctop, clen, cpar, ckoff, ckids, lvp,
-                          PATHS && npath ? pch : nullptr, nlev, P.vscale, singular);
+            bool good = P.axial_ok != 0;
+            for (int32_t i = tid; i < n; i += T) good &= good_divisor(sdr[i].x) && good_quotient(sdr[i].y);
+            if (__syncthreads_or(!good && !exact)) {   // assemble again, and divide
+                exact = true;
+                goto assemble;
+            }
+            exact = false;
+            for (int32_t i = tid; i < n; i += T) sv[i] = sv[i] + P.vscale * sdr[i].y;
         }
+        __syncthreads();
 
         // 8. cnexp state advance on the new voltage (time t + dt).
         for (int32_t g = 0; g < P.ngroups; ++g) {

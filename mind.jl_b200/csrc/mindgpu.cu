@@ -655,7 +655,7 @@ int create(const MindLayout *L, MindHandle *h) {
     std::vector<double> a(n), cdt(n), ad(n), v0(n);
     for (int64_t j = 0; j < n; ++j) {
         int32_t i = layout_of_packed[j];
-        a[j] = L->axial[i];
+        a[j] = parent[i] >= 0 ? L->axial[i] : 0.0;   // a root's is not used
         cdt[j] = L->capacitance[i] / (L->secondorder == 0 ? L->dt : 0.5 * L->dt);
         ad[j] = L->axial_diagonal[i];
         v0[j] = L->voltage[i];
@@ -924,6 +924,11 @@ int create(const MindLayout *L, MindHandle *h) {
     P.level_path = h->upload(level_path);
     P.path_off = h->upload(path_off);
     P.path_chain = h->upload(path_chain);
+    P.axial_ok = 1;
+    for (double x : a) {
+        const double m = std::fabs(x);
+        if (m != 0.0 && !(m >= 0x1p-480 && m < 0x1p480)) P.axial_ok = 0;
+    }
     P.part = h->upload(part);
     P.det_off = h->upload(det_off);
     P.det_node = h->upload(det_node);
