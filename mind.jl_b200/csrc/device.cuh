@@ -122,17 +122,19 @@ __host__ __device__ inline int kind_slots(int32_t kind) {
 /*
  * Rows whose state changes every step keep that state in shared memory for the
  * window; everything else of a row (parameters, decay factors) is streamed
- * from HBM.  hh rows are few per cell and keep all their slots on chip.
- *   staged_doubles  FP64 slots staged per row: hh all, ExpSyn g, Exp2Syn A,B.  State is
+ * from HBM.  hh rows also keep their seven parameters on chip, unless the launch is one of
+ * more cells than are resident at once and streaming them makes room for another
+ * (Params::hh_streamed).
+ *   staged_doubles  FP64 slots staged per row: hh m,h,n and its parameters, ExpSyn g, Exp2Syn A,B.  State is
  *                   FP64 in both modes; the mixed mode computes hh's rates and the
  *                   synapses' per-step decrements in FP32 and accumulates them in FP64.
  */
 __host__ __device__ inline bool kind_staged(int32_t kind) {
     return kind == MIND_MECH_HH || kind == MIND_MECH_EXPSYN || kind == MIND_MECH_EXP2SYN;
 }
-__host__ __device__ inline int staged_doubles(int32_t kind) {
+__host__ __device__ inline int staged_doubles(int32_t kind, bool hh_streamed) {
     switch (kind) {
-        case MIND_MECH_HH: return HH_NSLOT;
+        case MIND_MECH_HH: return hh_streamed ? 3 : 3 + HH_M;
         case MIND_MECH_EXPSYN: return 1;
         case MIND_MECH_EXP2SYN: return 2;
         default: return 0;
@@ -145,10 +147,9 @@ __host__ __device__ inline int staged_doubles(int32_t kind) {
  *            chain tops [nch each]; event increments [inbox_cap]; staged FP64
  *            slots of the staged rows;
  *   events   the cell's inbox for the window [inbox_cap];
- *   ints     per staged row: local node; chain top, length,
- *            parent, child-chain CSR; level starts; path starts; inbox
- *            order; the threads' row ranges per group [ngroups][threads + 1];
- *   shorts   chain of every node [n].
+ *   ints     chain top, length, parent, child-chain CSR; level starts; path starts; inbox order;
+ *   shorts   (words in an image in HBM) per staged row: local node; the threads' row ranges per
+ *            group [ngroups][threads + 1]; then, 16 bits in either, chain of every node [n].
  * Host (to size the launch) and device (to carve the buffer) use this one function.
  */
 struct CellShape {
@@ -157,17 +158,16 @@ struct CellShape {
 };
 
 __host__ __device__ inline size_t cell_smem_bytes(const CellShape &s, const int32_t *kinds, int32_t ngroups,
-                                                  int32_t inbox_cap) {
+                                                  int32_t inbox_cap, bool hbm, bool hh_streamed) {
     size_t doubles = 4 * (size_t)s.n + 6 + 2 * (size_t)s.nch + (size_t)inbox_cap;
-    size_t ints = 0;
+    size_t shorts = (size_t)ngroups * (kCellThreads + 1);
     for (int32_t g = 0; g < ngroups; ++g) {
         if (!kind_staged(kinds[g])) continue;
-        doubles += (size_t)staged_doubles(kinds[g]) * s.rows[g];
-        ints += (size_t)s.rows[g];
+        doubles += (size_t)staged_doubles(kinds[g], hh_streamed) * s.rows[g];
+        shorts += (size_t)s.rows[g];
     }
-    ints += 4 * (size_t)s.nch + 1 + (size_t)s.nkids + (size_t)s.nlev + 1 + (size_t)s.npath + 1 + (size_t)inbox_cap;
-    ints += (size_t)ngroups * (kCellThreads + 1);
-    return doubles * 8 + (size_t)inbox_cap * sizeof(InboxEvent) + ints * 4 + 2 * (size_t)s.n;
+    const size_t ints = 4 * (size_t)s.nch + 1 + (size_t)s.nkids + (size_t)s.nlev + 1 + (size_t)s.npath + 1 + (size_t)inbox_cap;
+    return doubles * 8 + (size_t)inbox_cap * sizeof(InboxEvent) + ints * 4 + shorts * (hbm ? 4 : 2) + 2 * (size_t)s.n;
 }
 
 struct Params {
@@ -206,6 +206,7 @@ struct Params {
     unsigned char *big_image;
     const int32_t *big_slot;
     int64_t big_stride;
+    int32_t hh_streamed;       // this launch reads hh parameters from HBM (staged_doubles)
     // detectors
     const int32_t *det_off;    // [ncells+1]
     const int32_t *det_node;   // local node

@@ -15,6 +15,8 @@
  */
 #pragma once
 
+#include <type_traits>
+
 #include "device.cuh"
 
 namespace mind {
@@ -466,11 +468,12 @@ __device__ __forceinline__ void sort_events(const InboxEvent *ev, int32_t m, int
     }
 }
 
-/* One mechanism group of the resident cell: staged state in shared memory, the rest in HBM. */
+/* One mechanism group of the resident cell: staged state in shared memory, the rest in HBM.  Local
+ * nodes take 16 bits in shared memory, 32 in an image in HBM. */
 struct StagedGroup {
     int32_t kind, rows, r0;   // r0 = first device row of the cell
     double *f;                // staged FP64 slots [slots][rows]
-    int32_t *node;            // local node per row
+    void *nodes;              // local node per row
     __device__ __forceinline__ double &at(int slot, int r) const { return f[slot * rows + r]; }
 };
 
@@ -707,16 +710,10 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
             sg[g].r0 = r0;
             sg[g].f = dp;
         }
-        if (staged) dp += (size_t)staged_doubles(G.kind) * rows;
+        if (staged) dp += (size_t)staged_doubles(G.kind, P.hh_streamed != 0) * rows;
     }
     InboxEvent *sev = reinterpret_cast<InboxEvent *>(dp);
     int32_t *ip = reinterpret_cast<int32_t *>(sev + P.inbox_cap);
-    for (int32_t g = 0; g < P.ngroups; ++g) {
-        const DevGroup &G = P.groups[g];
-        const int32_t rows = kind_staged(G.kind) ? G.row_off[c + 1] - G.row_off[c] : 0;
-        if (tid == 0) sg[g].node = ip;
-        ip += rows;
-    }
     int32_t *ctop = ip; ip += nch;
     int32_t *clen = ip; ip += nch;
     int32_t *cpar = ip; ip += nch;
@@ -725,8 +722,17 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     int32_t *lvp = ip; ip += nlev + 1;
     int32_t *pch = ip; ip += npath + 1;
     int32_t *sorder = ip; ip += P.inbox_cap;
-    int32_t *spart = ip; ip += P.ngroups * (O + 1);   // the threads' row ranges per group
-    int16_t *chain_of = reinterpret_cast<int16_t *>(ip);
+    using Index = typename std::conditional<GLOBAL_IMAGE, int32_t, uint16_t>::type;
+    Index *xp = reinterpret_cast<Index *>(ip);
+    for (int32_t g = 0; g < P.ngroups; ++g) {
+        const DevGroup &G = P.groups[g];
+        const int32_t rows = kind_staged(G.kind) ? G.row_off[c + 1] - G.row_off[c] : 0;
+        if (tid == 0) sg[g].nodes = xp;
+        xp += rows;
+    }
+    auto local_node = [](const StagedGroup &G, int32_t r) { return (int32_t) reinterpret_cast<const Index *>(G.nodes)[r]; };
+    Index *spart = xp; xp += P.ngroups * (O + 1);   // the threads' row ranges per group
+    int16_t *chain_of = reinterpret_cast<int16_t *>(xp);
     {
         // The launch sized the image for this cell's bin; refuse rather than overrun.
         uint32_t dynamic_bytes;
@@ -792,7 +798,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     for (int32_t k = tid; k < nkids; k += T) ckids[k] = P.chain_kids[kb + k];
     for (int32_t k = tid; k <= nlev; k += T) lvp[k] = P.level_path[lv0 + k];
     for (int32_t k = tid; k <= npath; k += T) pch[k] = P.path_chain[pb + k];
-    for (int32_t k = tid; k < P.ngroups * (O + 1); k += T) spart[k] = P.part[(int64_t)c * P.ngroups * (O + 1) + k];
+    for (int32_t k = tid; k < P.ngroups * (O + 1); k += T) spart[k] = (Index)P.part[(int64_t)c * P.ngroups * (O + 1) + k];
     __syncthreads();
     for (int32_t k = tid; k < nch; k += T)
         for (int32_t i = ctop[k]; i < ctop[k] + clen[k]; ++i) chain_of[i] = (int16_t)k;
@@ -804,7 +810,9 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
             const int32_t row = S.r0 + r;
             switch (S.kind) {
                 case MIND_MECH_HH:
-                    for (int k = 0; k < HH_NSLOT; ++k) S.at(k, r) = G.f[k][row];
+                    for (int k = 0; k < 3; ++k) S.at(k, r) = G.f[HH_M + k][row];
+                    if (!P.hh_streamed)
+                        for (int k = 0; k < HH_M; ++k) S.at(3 + k, r) = G.f[k][row];
                     break;
                 case MIND_MECH_EXPSYN:
                     S.at(0, r) = G.f[ES_G][row];
@@ -814,7 +822,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     S.at(1, r) = G.f[E2_B][row];
                     break;
             }
-            S.node[r] = (int32_t)(G.node[row] - nb);
+            reinterpret_cast<Index *>(S.nodes)[r] = (Index)(G.node[row] - nb);
         }
     }
     // Detectors stay in registers for the window (at most one per lane; checked at mind_create).
@@ -1005,27 +1013,26 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     }
                 } else if (G.kind == MIND_MECH_HH) {
                     for (int32_t r = lo; r < hi; ++r) {
-                        const int32_t node = G.node[r];
+                        const int64_t q = (int64_t)G.r0 + r;
+                        auto parameter = [&](int k) { return P.hh_streamed ? __ldg(GG.f[k] + q) : G.at(3 + k, r); };
+                        const double gnabar = parameter(HH_GNABAR), gkbar = parameter(HH_GKBAR), gl = parameter(HH_GL);
+                        const double el = parameter(HH_EL), ena = parameter(HH_ENA), ek = parameter(HH_EK);
+                        const double scale = parameter(HH_SCALE);
+                        const int32_t node = local_node(G, r);
                         const double vv = sv[node];
                         const double probe = vv + 0.001;
-                        const double m = G.at(HH_M, r), h = G.at(HH_H, r), nn = G.at(HH_N, r);
+                        const double m = G.at(0, r), h = G.at(1, r), nn = G.at(2, r);
                         if (MIXED) {
                             // at fixed gates the current is linear in v: dI/dv is the summed conductance
-                            const double gna = G.at(HH_GNABAR, r) * m * m * m * h;
-                            const double gk = G.at(HH_GKBAR, r) * nn * nn * nn * nn;
-                            const double gl = G.at(HH_GL, r);
-                            const double i = gl * (vv - G.at(HH_EL, r)) + gna * (vv - G.at(HH_ENA, r)) +
-                                             gk * (vv - G.at(HH_EK, r));
-                            const double scale = G.at(HH_SCALE, r);
+                            const double gna = gnabar * m * m * m * h;
+                            const double gk = gkbar * nn * nn * nn * nn;
+                            const double i = gl * (vv - el) + gna * (vv - ena) + gk * (vv - ek);
                             sdr[node].y = sdr[node].y - scale * i;
                             sdr[node].x = sdr[node].x + scale * (gna + gk + gl);
                             continue;
                         }
-                        const double shifted = hh_current(probe, m, h, nn, G.at(HH_GNABAR, r), G.at(HH_GKBAR, r),
-                                                          G.at(HH_GL, r), G.at(HH_EL, r), G.at(HH_ENA, r), G.at(HH_EK, r));
-                        const double value = hh_current(vv, m, h, nn, G.at(HH_GNABAR, r), G.at(HH_GKBAR, r),
-                                                        G.at(HH_GL, r), G.at(HH_EL, r), G.at(HH_ENA, r), G.at(HH_EK, r));
-                        const double scale = G.at(HH_SCALE, r);
+                        const double shifted = hh_current(probe, m, h, nn, gnabar, gkbar, gl, el, ena, ek);
+                        const double value = hh_current(vv, m, h, nn, gnabar, gkbar, gl, el, ena, ek);
                         sdr[node].y = sdr[node].y - scale * value;
                         sdr[node].x = sdr[node].x + milli_quotient<MIXED>(scale * (shifted - value));
                     }
@@ -1033,7 +1040,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     const bool two = G.kind == MIND_MECH_EXP2SYN;
                     const double *pe = GG.f[two ? E2_E : ES_E] + G.r0;
                     for (int32_t r = lo; r < hi; ++r) {
-                        const int32_t node = G.node[r];
+                        const int32_t node = local_node(G, r);
                         const double e = __ldg(pe + r);
                         double gs;
                         if (two)
@@ -1132,17 +1139,16 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     for (int32_t w = tid; w < 3 * lanes; w += T) {
                         const int32_t gate = (w >= lanes) + (w >= 2 * lanes), r = w - gate * lanes;
                         if (r >= G.rows) continue;
-                        const double vv = sv[G.node[r]];
-                        const int slot = HH_M + gate;
-                        const double state = G.at(slot, r);
+                        const double vv = sv[local_node(G, r)];
+                        const double state = G.at(gate, r);
                         if (MIXED) {
                             float inf, factor;
                             hh_gate_f32(vv, q10f, (float)P.dt, gate, inf, factor);
-                            G.at(slot, r) = state + (double)factor * ((double)inf - state);
+                            G.at(gate, r) = state + (double)factor * ((double)inf - state);
                         } else {
                             double inf, tau;
                             hh_gate(vv, q10, gate, inf, tau);
-                            G.at(slot, r) = cnexp(state, inf, tau, P.dt);
+                            G.at(gate, r) = cnexp(state, inf, tau, P.dt);
                         }
                     }
                 } break;
@@ -1209,10 +1215,10 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
             const int32_t row = S.r0 + r;
             switch (S.kind) {
                 case MIND_MECH_HH:
-                    G.f[HH_M][row] = S.at(HH_M, r);
-                    G.f[HH_H][row] = S.at(HH_H, r);
-                    G.f[HH_N][row] = S.at(HH_N, r);
-                    finite &= isfinite(S.at(HH_M, r)) && isfinite(S.at(HH_H, r)) && isfinite(S.at(HH_N, r));
+                    for (int k = 0; k < 3; ++k) {
+                        G.f[HH_M + k][row] = S.at(k, r);
+                        finite &= isfinite(S.at(k, r));
+                    }
                     break;
                 case MIND_MECH_EXPSYN:
                     G.f[ES_G][row] = S.at(0, r);

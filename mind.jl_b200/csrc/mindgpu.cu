@@ -175,6 +175,7 @@ struct MindHandle {
         int32_t max_detectors = 0;        // most threshold detectors on one of its cells
         bool global_image = false;        // cells too large for shared memory: image in HBM
         bool paths = false;               // some cell has the path schedule of the solve
+        bool hh_streamed = false;         // hh parameters are read from HBM
     };
     std::vector<Bin> bins;           // cells grouped by shared-memory need
     std::vector<cudaStream_t> bin_streams;   // size bins run concurrently
@@ -397,7 +398,7 @@ int readable_slot(int32_t kind, const char *name) {
 /* Index of a device slot in a group's staged shared-memory rows, or -1 (read from HBM). */
 int staged_slot(int32_t kind, int slot) {
     switch (kind) {
-        case MIND_MECH_HH: return slot;
+        case MIND_MECH_HH: return slot >= HH_M && slot <= HH_N ? slot - HH_M : -1;
         case MIND_MECH_EXPSYN: return slot == ES_G ? 0 : -1;
         case MIND_MECH_EXP2SYN: return slot == E2_A ? 0 : slot == E2_B ? 1 : -1;
         default: return -1;
@@ -427,6 +428,12 @@ cudaError_t set_window_smem(int bytes) {
  * leaves room for more resident CTAs per SM than the default register bound (228 KB per SM,
  * 1 KB reserved per CTA). */
 bool tight_by_default(size_t smem_bytes) { return (smem_bytes + 1024) * 6 <= 228 * 1024; }
+
+/* Cells of an image size that one multiprocessor holds, up to the register bounds of the launch
+ * shapes. */
+int64_t resident_cells(size_t smem_bytes) {
+    return std::min<int64_t>(kTightBlocks, (int64_t)(228 * 1024 / (smem_bytes + 1024)));
+}
 
 bool valid_cell_threads(int32_t threads) {
     return threads == kCellThreads || threads == kCellThreads / 2 || threads == kCellThreads / 4;
@@ -990,7 +997,11 @@ int create(const MindLayout *L, MindHandle *h) {
         for (int32_t r = 0; r < (int32_t)row_cell[g].size(); ++r) group_row_off[g][row_cell[g][r] + 1]++;
         for (int32_t c = 0; c < ncells; ++c) group_row_off[g][c + 1] += group_row_off[g][c];
     }
+    // A cell whose image exceeds what one CTA can add to the kernel's static shared memory
+    // keeps its image in an HBM slot (one bin, launched without dynamic shared memory).
+    const size_t smem_limit = 227 * 1024 - 1024;
     std::vector<std::pair<size_t, int32_t>> need(ncells);
+    std::vector<size_t> lean_bytes(ncells, 0);   // with hh parameters streamed
     size_t worst_any = 0;
     for (int32_t c = 0; c < ncells; ++c) {
         CellShape shape{};
@@ -1002,14 +1013,17 @@ int create(const MindLayout *L, MindHandle *h) {
         shape.nlev = level_off[c + 1] - level_off[c] - 1;
         shape.npath = path_off[c + 1] - path_off[c] - 1;
         for (int32_t g = 0; g < L->n_mechanisms; ++g) shape.rows[g] = group_row_off[g][c + 1] - group_row_off[g][c];
-        const size_t bytes = cell_smem_bytes(shape, kinds.data(), L->n_mechanisms, P.inbox_cap);
+        size_t bytes = cell_smem_bytes(shape, kinds.data(), L->n_mechanisms, P.inbox_cap, false, false);
+        lean_bytes[c] = cell_smem_bytes(shape, kinds.data(), L->n_mechanisms, P.inbox_cap, false, true);
+        // row ranges take 16 bits in shared memory
+        bool fits = bytes <= smem_limit;
+        for (int32_t g = 0; g < L->n_mechanisms; ++g) fits = fits && shape.rows[g] <= 65535;
+        if (!fits)
+            bytes = std::max(smem_limit + 1, cell_smem_bytes(shape, kinds.data(), L->n_mechanisms, P.inbox_cap, true, false));
         need[c] = {bytes, c};
         worst_any = std::max(worst_any, bytes);
     }
     std::stable_sort(need.begin(), need.end(), [](const auto &x, const auto &y) { return x.first > y.first; });
-    // A cell whose image exceeds what one CTA can add to the kernel's static shared memory
-    // keeps its image in an HBM slot (one bin, launched without dynamic shared memory).
-    const size_t smem_limit = 227 * 1024 - 1024;
     size_t n_big = 0, big_bytes = 0;
     while (n_big < need.size() && need[n_big].first > smem_limit) big_bytes = std::max(big_bytes, need[n_big++].first);
     std::vector<int32_t> big_slot(ncells, -1);
@@ -1017,23 +1031,44 @@ int create(const MindLayout *L, MindHandle *h) {
     for (size_t k = 0; k < n_big; ++k) big_slot[need[k].second] = (int32_t)k;
     P.big_image = n_big ? h->alloc<unsigned char>(n_big * (size_t)P.big_stride) : nullptr;
     P.big_slot = h->upload(big_slot);
+    // A network whose cells are all resident at once is one launch: there is nothing to gain from
+    // matching launches to sizes, and one launch spreads evenly over the multiprocessors (250
+    // pyramidal cells, FP64: 77 us per step in two launches, 64 in one).  Blocks go to the
+    // multiprocessors in turn, so a round of smallest-first and one of largest-first alternate and
+    // the largest cells share theirs with the fewest and smallest others.
+    constexpr int32_t kProcessors = 148;
+    const bool resident = n_big == 0 && ncells > 0 && ncells <= kProcessors * resident_cells(need[0].first);
+    const size_t largest = ncells > 0 ? need[0].first : 0;
+    if (resident)
+        for (int32_t k = 0; k < ncells; k += 2 * kProcessors)
+            std::reverse(need.begin() + k, need.begin() + std::min(ncells, k + kProcessors));
     size_t worst_smem = 0;
     std::vector<int32_t> bin_cells;
     for (size_t k = 0; k < need.size();) {
-        size_t top = need[k].first;
+        size_t top = resident ? largest : need[k].first;
         size_t first = k;
         const bool big = k < n_big;
         if (big)
             k = n_big;
         else
-            while (k < need.size() && need[k].first * 4 >= top * 3) ++k;
+            while (k < need.size() && (resident || need[k].first * 3 >= top * 2)) ++k;
         MindHandle::Bin bin;
         bin.first = (int32_t)first;
         bin.count = (int32_t)(k - first);
         bin.smem_bytes = big ? 0 : top;
         bin.global_image = big;
-        bin.tight = !big && tight_by_default(top);
-        if (!big) worst_smem = std::max(worst_smem, top);
+        if (!big) {
+            // Streaming the hh parameters costs a few hundred cycles of a step (1,000 cells of
+            // 300-600 compartments: 23 -> 25 us per step); it pays where it lets another cell onto a
+            // multiprocessor and there are more cells than places (1,000 pyramidal cells of
+            // 700-1,200 compartments, mixed: 70 -> 52 us per step, three cells -> four).
+            size_t lean = 0;
+            for (size_t q = first; q < k; ++q) lean = std::max(lean, lean_bytes[need[q].second]);
+            bin.hh_streamed = (int64_t)ncells > 148 * resident_cells(top) && resident_cells(lean) > resident_cells(top);
+            if (bin.hh_streamed) bin.smem_bytes = lean;
+        }
+        bin.tight = !big && tight_by_default(bin.smem_bytes);
+        if (!big) worst_smem = std::max(worst_smem, bin.smem_bytes);
         for (size_t q = first; q < k; ++q) {
             bin.max_detectors = std::max(bin.max_detectors, det_off[need[q].second + 1] - det_off[need[q].second]);
             bin.paths = bin.paths || cell_paths[need[q].second];
@@ -1460,6 +1495,7 @@ int advance(MindHandle *h, int64_t steps, bool record_spikes) {
             cudaStream_t s = h->bin_streams[b];
             cudaStreamWaitEvent(s, h->fork, 0);
             const int32_t *cells = h->bin_cells + bin.first;
+            P.hh_streamed = bin.hh_streamed ? 1 : 0;
             if (h->precision == MIND_MIXED)
                 launch_window<true>(h, bin, s, P, cells, n0, W);
             else
