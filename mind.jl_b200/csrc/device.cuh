@@ -9,8 +9,8 @@
  *     nodes contiguous from top to bottom.  A cell is staged in shared memory
  *     once per window of steps.
  *   - Mechanism rows are structure-of-arrays per group, sorted by
- *     (cell, owner thread = local node mod 64, local node, layout row): a cell
- *     owns one contiguous row range per group, each thread of its CTA one
+ *     (cell, owner slot = local node mod 128, local node, layout row): a cell
+ *     owns one contiguous row range per group, each owner slot one
  *     sub-range, and rows on one node are adjacent (a "segment").
  *   - Events live in a ring of delivery bins (bin m = the events NEURON's two
  *     half-step deliveries hand to step m's currents, i.e. event times in
@@ -47,10 +47,10 @@ constexpr int kCellThreads = 128;  // window kernel: one cell per CTA of four wa
 // A 128-thread window launch whose cells need little shared memory can keep more CTAs per SM
 // than its registers allow at the default bound (5): the tight variant is compiled for 7.
 constexpr int kTightBlocks = 7;
-// CTAs per SM a launch shape is compiled for by default (its __launch_bounds__): 5 at 128
-// threads per cell, 10 at 64, 16 at one warp.
+// CTAs per SM a launch shape is compiled for by default (its __launch_bounds__): 2 at 256
+// threads per cell, 5 at 128, 10 at 64, 16 at one warp.
 constexpr int default_min_blocks(int threads) {
-    return threads == kCellThreads ? 5 : threads == kCellThreads / 2 ? 10 : 16;
+    return threads == 2 * kCellThreads ? 2 : threads == kCellThreads ? 5 : threads == kCellThreads / 2 ? 10 : 16;
 }
 constexpr int kSurrogateRing = 21;  // drive bins kept for the surrogate: the last 20 and the current
 
@@ -87,6 +87,7 @@ struct DevGroup {
     double *cols;
     int32_t ncols;
     int32_t gen;              // index into kGenMechanisms, -1 for the hand-written kinds
+    int32_t part;             // place among the groups of Params::part, -1 for artificial cells
 };
 
 __host__ __device__ inline bool kind_generated(int32_t kind) {
@@ -129,6 +130,10 @@ __host__ __device__ inline int kind_slots(int32_t kind) {
  *                   FP64 in both modes; the mixed mode computes hh's rates and the
  *                   synapses' per-step decrements in FP32 and accumulates them in FP64.
  */
+/* Whether rows of the kind sit on nodes (artificial cells' do not). */
+__host__ __device__ inline bool kind_placed(int32_t kind) {
+    return kind != MIND_MECH_NETSTIM && kind != MIND_MECH_PATTERNSTIM;
+}
 __host__ __device__ inline bool kind_staged(int32_t kind) {
     return kind == MIND_MECH_HH || kind == MIND_MECH_EXPSYN || kind == MIND_MECH_EXP2SYN;
 }
@@ -149,7 +154,7 @@ __host__ __device__ inline int staged_doubles(int32_t kind, bool hh_streamed) {
  *   events   the cell's inbox for the window [inbox_cap];
  *   ints     chain top, length, parent, child-chain CSR; level starts; path starts; inbox order;
  *   shorts   (words in an image in HBM) per staged row: local node; the threads' row ranges per
- *            group [ngroups][threads + 1]; then, 16 bits in either, chain of every node [n].
+ *            placed group [owner slots + 1]; then, 16 bits in either, chain of every node [n].
  * Host (to size the launch) and device (to carve the buffer) use this one function.
  */
 struct CellShape {
@@ -160,8 +165,9 @@ struct CellShape {
 __host__ __device__ inline size_t cell_smem_bytes(const CellShape &s, const int32_t *kinds, int32_t ngroups,
                                                   int32_t inbox_cap, bool hbm, bool hh_streamed) {
     size_t doubles = 4 * (size_t)s.n + 6 + 2 * (size_t)s.nch + (size_t)inbox_cap;
-    size_t shorts = (size_t)ngroups * (kCellThreads + 1);
+    size_t shorts = 0;
     for (int32_t g = 0; g < ngroups; ++g) {
+        if (kind_placed(kinds[g])) shorts += kCellThreads + 1;
         if (!kind_staged(kinds[g])) continue;
         doubles += (size_t)staged_doubles(kinds[g], hh_streamed) * s.rows[g];
         shorts += (size_t)s.rows[g];
@@ -198,9 +204,11 @@ struct Params {
                                  // cell on the chain schedule (its paths are its chains)
     int32_t axial_ok;          // every axial conductance is 0 or in [2^-480, 2^480)
     DevGroup groups[kMaxGroups];
-    // per cell, group and thread: first row (relative to the cell's first row of the group)
-    // of the thread's rows; thread t owns the local nodes i with i % kCellThreads == t
-    const int32_t *part;       // [ncells][ngroups][kCellThreads + 1]
+    // per cell, placed group and owner slot: first row (relative to the cell's first row of the group)
+    // of the owner's rows; owner slot t holds the local nodes i with
+    // i % kCellThreads == t
+    const int32_t *part;       // [ncells][nparts][kCellThreads + 1]
+    int32_t nparts;            // groups whose rows sit on nodes
     // cells whose image exceeds a CTA's shared memory keep it in HBM: slot big_slot[c] of
     // big_image, big_stride bytes each (big_slot -1 for the others)
     unsigned char *big_image;

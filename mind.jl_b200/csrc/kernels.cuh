@@ -654,7 +654,7 @@ __device__ __forceinline__ void hines(double2 *sdr, const double *sa, double *sx
 }
 
 /*
- * One CTA of four warps advances one cell through W micro steps.  Shared memory
+ * One CTA advances one cell through W micro steps.  Shared memory
  * holds what the serial parts of the step touch: v, d, rhs and axial
  * conductance of every node, the chain tables of the Hines solve, the state
  * that changes every step (hh gates, synaptic conductances) and the window's
@@ -675,7 +675,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     const int32_t tid = threadIdx.x;
     constexpr int32_t T = NT;            // threads of this launch
     constexpr int32_t O = kCellThreads;  // owner slots: node i belongs to slot i % O
-    static_assert(O % T == 0, "a thread serves whole owner slots");
+    static_assert(O % T == 0 || T == 2 * O, "a thread serves whole owner slots, or two threads one");
     const int64_t nb = P.node_off[c];
     const int32_t n = (int32_t)(P.node_off[c + 1] - nb);
     const int32_t cb = P.chain_off[c];
@@ -731,7 +731,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
         xp += rows;
     }
     auto local_node = [](const StagedGroup &G, int32_t r) { return (int32_t) reinterpret_cast<const Index *>(G.nodes)[r]; };
-    Index *spart = xp; xp += P.ngroups * (O + 1);   // the threads' row ranges per group
+    Index *spart = xp; xp += P.nparts * (O + 1);   // the owners' row ranges per group
     int16_t *chain_of = reinterpret_cast<int16_t *>(xp);
     {
         // The launch sized the image for this cell's bin; refuse rather than overrun.
@@ -798,7 +798,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     for (int32_t k = tid; k < nkids; k += T) ckids[k] = P.chain_kids[kb + k];
     for (int32_t k = tid; k <= nlev; k += T) lvp[k] = P.level_path[lv0 + k];
     for (int32_t k = tid; k <= npath; k += T) pch[k] = P.path_chain[pb + k];
-    for (int32_t k = tid; k < P.ngroups * (O + 1); k += T) spart[k] = (Index)P.part[(int64_t)c * P.ngroups * (O + 1) + k];
+    for (int32_t k = tid; k < P.nparts * (O + 1); k += T) spart[k] = (Index)P.part[(int64_t)c * P.nparts * (O + 1) + k];
     __syncthreads();
     for (int32_t k = tid; k < nch; k += T)
         for (int32_t i = ctop[k]; i < ctop[k] + clen[k]; ++i) chain_of[i] = (int16_t)k;
@@ -941,12 +941,28 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
         for (int32_t i = tid; i < n; i += T) {
             sdr[i] = make_double2(0.0, 0.0);
         }
+        //      Where two threads share a slot, they halve the rows of the density groups (one per
+        //      node), the first takes those of the others, and barriers stand between.
+        constexpr bool kShared = T > O;
+        bool unsynced = false;   // rows of a group that was not halved may be in flight
+        if (kShared) __syncthreads();
         const double tc = t + 0.5 * P.dt;
         for (int32_t g = 0; g < P.ngroups; ++g) {
             const DevGroup &GG = P.groups[g];
             const StagedGroup G = sg[g];
-            for (int32_t slot = tid; slot < O; slot += T) {
-                const int32_t lo = spart[g * (O + 1) + slot], hi = spart[g * (O + 1) + slot + 1];
+            if (GG.part < 0) continue;
+            const bool halved = kShared && (G.kind == MIND_MECH_PAS || G.kind == MIND_MECH_HH);
+            if (halved && unsynced) __syncthreads();
+            unsynced = !halved;
+            for (int32_t slot = kShared ? tid % O : tid; slot < O; slot += T) {
+                int32_t lo = spart[GG.part * (O + 1) + slot], hi = spart[GG.part * (O + 1) + slot + 1];
+                if (kShared) {
+                    const int32_t middle = halved ? (lo + hi + 1) / 2 : hi;
+                    if (tid < O)
+                        hi = middle;
+                    else
+                        lo = middle;
+                }
                 if (lo >= hi) continue;
                 if (G.kind == MIND_MECH_PAS) {
                     if (MIXED) continue;  // folded into the node constants of the assembly below
@@ -1061,7 +1077,9 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     }
                 }
             }
+            if (halved) __syncthreads();
         }
+        if (kShared) __syncthreads();
         // Cable assembly of the owned nodes: d = C/dt + d + axial_diagonal; own axial term, then children.
         for (int32_t i = tid; i < n; i += T) {
             const int64_t gi = nb + i;

@@ -170,9 +170,10 @@ struct MindHandle {
     struct Bin {
         int32_t first, count;
         size_t smem_bytes;
-        int32_t threads = kCellThreads;   // CTA size of the bin's launches (kCellThreads or half)
+        int32_t threads = kCellThreads;   // launch shape: kCellThreads, half or a quarter
         bool tight = false;               // 128 threads, compiled for kTightBlocks CTAs per SM
         int32_t max_detectors = 0;        // most threshold detectors on one of its cells
+        int32_t max_nodes = 0;            // most nodes of one of its cells
         bool global_image = false;        // cells too large for shared memory: image in HBM
         bool paths = false;               // some cell has the path schedule of the solve
         bool hh_streamed = false;         // hh parameters are read from HBM
@@ -413,6 +414,7 @@ int launch_grid(int64_t work) {
 }
 
 /* The window kernel's launch shapes: 128 threads per cell (kCellThreads), 64, or one warp;
+ * 256 where the 128-thread shape has room (`twice` in launch_window);
  * the 128-thread shapes also without the path schedule (PATHS false). */
 template <int NT, int MINB = default_min_blocks(NT), bool PATHS = true>
 cudaError_t set_window_smem(int bytes) {
@@ -681,11 +683,13 @@ int create(const MindLayout *L, MindHandle *h) {
     std::vector<std::vector<int32_t>> &dev_row_of = h->dev_row_of;  // layout row -> device row
     dev_row_of.assign(L->n_mechanisms, {});
     h->field_slot.assign(L->n_mechanisms, {});
-    // Thread t of a cell's CTA owns the local nodes i with i % kCellThreads == t, so that the
+    // Owner slot t of a cell holds the local nodes i with i % kCellThreads == t, so that the
     // threads of a warp touch consecutive nodes (distinct shared-memory banks).  Each
     // group's rows are sorted by (cell, owner thread, node, layout row): a thread's rows are
     // one range, and rows of one node stay in layout order.
-    std::vector<int32_t> part((size_t)ncells * L->n_mechanisms * (kCellThreads + 1), 0);
+    for (int32_t g = 0; g < L->n_mechanisms; ++g)
+        P.groups[g].part = kind_placed(L->mechanisms[g].kind) ? P.nparts++ : -1;
+    std::vector<int32_t> part((size_t)ncells * P.nparts * (kCellThreads + 1), 0);
     // Mixed mode folds pas into per-node constants: its conductance g*area*0.01 and
     // that times e (the probe's (i(v+0.001)-i(v))/0.001 of a linear current is g).
     std::vector<double> mix_gs(n, 0.0), mix_gse(n, 0.0);
@@ -782,7 +786,7 @@ int create(const MindLayout *L, MindHandle *h) {
             for (int32_t c = 0; c < ncells; ++c) row_off[c + 1] += row_off[c];
             // thread t's rows: the range after the rows of the owners before it
             for (int32_t c = 0; c < ncells; ++c) {
-                int32_t *pc = part.data() + ((size_t)c * L->n_mechanisms + g) * (kCellThreads + 1);
+                int32_t *pc = part.data() + ((size_t)c * P.nparts + P.groups[g].part) * (kCellThreads + 1);
                 for (int32_t r = row_off[c]; r < row_off[c + 1]; ++r)
                     pc[(node_dev[r] - node_off[c]) % kCellThreads + 1]++;
                 for (int32_t t = 0; t < kCellThreads; ++t) pc[t + 1] += pc[t];
@@ -1072,6 +1076,7 @@ int create(const MindLayout *L, MindHandle *h) {
         for (size_t q = first; q < k; ++q) {
             bin.max_detectors = std::max(bin.max_detectors, det_off[need[q].second + 1] - det_off[need[q].second]);
             bin.paths = bin.paths || cell_paths[need[q].second];
+            bin.max_nodes = std::max(bin.max_nodes, (int32_t)(node_off[need[q].second + 1] - node_off[need[q].second]));
         }
         h->bins.push_back(bin);
     }
@@ -1096,6 +1101,11 @@ int create(const MindLayout *L, MindHandle *h) {
     CUDA_TRY(h, cudaFuncSetAttribute(window_kernel<false, kCellThreads, false, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr));
     CUDA_TRY(h, cudaFuncSetAttribute(window_kernel<true, kCellThreads, false, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr));
+    CUDA_TRY(h, set_window_smem<2 * kCellThreads>(smem_attr));
+    CUDA_TRY(h, cudaFuncSetAttribute(window_kernel<false, 2 * kCellThreads, false, true>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr));
+    CUDA_TRY(h, cudaFuncSetAttribute(window_kernel<true, 2 * kCellThreads, false, true>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, smem_attr));
     CUDA_TRY(h, set_window_smem<kCellThreads / 2>(smem_attr));
     CUDA_TRY(h, set_window_smem<kCellThreads / 4>(smem_attr));
@@ -1350,17 +1360,28 @@ void launch_window(const MindHandle *h, const MindHandle::Bin &bin, cudaStream_t
                    const int32_t *cells, int64_t n0, int32_t W) {
     constexpr int T = kCellThreads;
     const size_t smem = bin.smem_bytes;
+    // The 128-thread shape takes 256 threads per cell where there is room for it: at most two cells
+    // per multiprocessor (detailed ones; a surrogate's cells only sum their events), more nodes
+    // than 128 threads take in one go.  The sweeps are as long, most of the rest is halved (us per
+    // step, 128 -> 256 threads: 61 trees 36.0 -> 35.1, 250 pyramidal cells 62.7 -> 58.5, 151 clamped
+    // ones 67.4 -> 62.2, 20 detailed among 1,000 surrogate cells 20.7 -> 19.3).  Networks of
+    // more cells fill their registers with cells instead.
+    const bool twice = bin.threads == T && !bin.global_image && bin.max_nodes > T && h->ncells - h->n_sur <= 2 * 148;
     if (h->gen_runtime) {   // the same kernel from a module compiled at run time
         const void *k = (const void *)h->rt_window[MIXED ? 1 : 0][bin.global_image ? 1 : 0];
         void *args[] = {(void *)&P, (void *)&cells, (void *)&n0, (void *)&W};
         cudaLaunchKernel(k, dim3(bin.count), dim3(T), args, bin.global_image ? 0 : smem, s);
-    } else if (h->has_generated) {   // mechanisms emitted from MOD files: the variant that runs them, 128 threads
+    } else if (h->has_generated) {   // mechanisms emitted from MOD files: the variant that runs them
         if (bin.global_image)
             window_kernel<MIXED, T, true, true><<<bin.count, T, 0, s>>>(P, cells, n0, W);
+        else if (twice)
+            window_kernel<MIXED, 2 * T, false, true><<<bin.count, 2 * T, smem, s>>>(P, cells, n0, W);
         else
             window_kernel<MIXED, T, false, true><<<bin.count, T, smem, s>>>(P, cells, n0, W);
     } else if (bin.global_image)
         window_kernel<MIXED, T, true><<<bin.count, T, 0, s>>>(P, cells, n0, W);
+    else if (twice)
+        window_kernel<MIXED, 2 * T><<<bin.count, 2 * T, smem, s>>>(P, cells, n0, W);
     else if (bin.threads == T && bin.tight && bin.paths)
         window_kernel<MIXED, T, false, false, kTightBlocks><<<bin.count, T, smem, s>>>(P, cells, n0, W);
     else if (bin.threads == T && bin.tight)
@@ -2168,7 +2189,7 @@ int mind_autotune(MindHandle *h, int32_t windows) {
     const std::pair<int32_t, bool> shapes[4] = {
         {kCellThreads, false}, {kCellThreads, true}, {kCellThreads / 2, false}, {kCellThreads / 4, false}};
     for (auto &bin : h->bins) {
-        if (bin.global_image || h->has_generated) continue;   // HBM images and emitted mechanisms: 128 threads
+        if (bin.global_image || h->has_generated) continue;   // HBM images and emitted mechanisms: one shape
         const std::pair<int32_t, bool> keep{bin.threads, bin.tight};
         for (const auto &shape : shapes) {
             if (shape == keep || shape.first < bin.max_detectors) continue;   // one detector per thread

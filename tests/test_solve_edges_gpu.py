@@ -80,3 +80,30 @@ def test_solve_equals_the_oracle(shape, change):
     # mixed: FP32 gating (bound of the mixed mode's own parity tests over a spike)
     mixed, _ = _run(layout, "mixed", steps, nodes)
     assert np.max(np.abs(mixed - ref.trace)) < 0.1
+
+
+def test_256_threads_per_cell_equal_64():
+    """A small network runs 256 threads per cell, two on an owner slot; asked for 64 threads, two
+    slots on one.  hh and pas share the soma here, in both orders, with synapses on top."""
+    for first, second in (("hh", "pas"), ("pas", "hh")):
+        model = mb.MicroModel(celsius=6.3)
+        secs = _sections("bush")
+        for k, cell in enumerate(mb.add_population(model, secs, 5, voltage=-65.0)):
+            mb.insert(cell, mb.builtin(first))
+            mb.insert(cell, mb.builtin(second), sections="soma" if second == "pas" else "dend")
+            mb.register_spike_source(cell, threshold=-10.0)
+            mb.add_pointprocess(cell, mb.builtin("IClamp"), section="d9", params={"del": 0.2, "dur": 3.0, "amp": 0.2 + 0.1 * k})
+            mb.add_pointprocess(cell, mb.builtin("AlphaSynapse"), section="d9", params={"onset": 0.5, "tau": 1.0, "gmax": 0.01})
+        layout = mb.build(model)
+        steps = 160
+        nodes = np.unique(np.linspace(1, layout.n_nodes, 15).astype(int))
+        ref = oracle.run(layout, steps, nodes)
+        assert ref.status == 0, ref.message
+        records = [mb.RecordSpec(int(n), f"n{n}") for n in nodes]
+        for threads in (128, 64):
+            state = DeviceState(layout, "fp64")
+            state.set_bin_threads([threads] * len(state.bin_threads()))
+            state.initialize()
+            trace = state.run_steps(steps, records).traces.by_record.T
+            state.close()
+            assert np.array_equal(trace, ref.trace), (first, threads, float(np.max(np.abs(trace - ref.trace))))
