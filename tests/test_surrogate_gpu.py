@@ -230,3 +230,29 @@ def test_rotating_judge_sample_sees_more_cells_and_still_reverts_a_failing_surro
     state.close()
     net.close()
     net2.close()
+
+
+@pytest.mark.parametrize("layers,hidden,rows", [(1, 16, 33), (2, 256, 700), (6, 64, 2500)])
+def test_gradients_on_side_streams_repeat_bit_for_bit(layers, hidden, rows):
+    """The backward pass runs its parameter gradients beside the chain of dz products, whose two
+    buffers take turns: repeated gradients and repeated trainings are the same bits, and the
+    gradient is the oracle's within the BF16 bounds of the tests above."""
+    rng = np.random.default_rng(layers)
+    x = rng.normal(0.0, 1.0, (rows, 70)).astype(np.float32)
+    y = (rng.uniform(size=rows) < 0.3).astype(np.float32)
+    net = surrogate.Mlp(n_in=70, hidden=hidden, layers=layers, seed=8)
+    want_loss, want = oracle_mlp.loss_and_gradients(net.params.astype(np.float64), [70] + [hidden] * layers + [1], x, y)
+    first, loss = net.gradients(x, y)
+    assert np.linalg.norm(first - want) / np.linalg.norm(want) < 5e-2
+    assert abs(loss - want_loss) < 1e-2 * want_loss
+    for _ in range(20):
+        again, _ = net.gradients(x, y)
+        assert np.array_equal(again, first)
+    net.close()
+    runs = []
+    for _ in range(2):
+        net = surrogate.Mlp(n_in=70, hidden=hidden, layers=layers, seed=8)
+        losses, _ = net.train(x, y, steps=30, batch=rows)
+        runs.append((losses, net.params))
+        net.close()
+    assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
