@@ -15,12 +15,13 @@
  *     them before anything leaves the SM:
  *       EPI_HIDDEN  z = acc + b, h = SiLU(z): z (FP32, for the backward pass), h as BF16 rows
  *                   and, for the weight gradients, as BF16 columns (h transposed);
- *       EPI_HEAD    the last hidden map with the 1-wide output map folded in (the tile spans
- *                   every column): logit = b_out + sum_n SiLU(acc + b)_n w_out[n]; inference
- *                   writes sigmoid(logit); training writes the row's sigmoid cross-entropy,
- *                   dlogit = (sigmoid - y) / rows, SiLU(z) transposed, and the gradient of
- *                   the hidden map's pre-activation dz = dlogit w_out SiLU'(z) as BF16 rows
- *                   and columns;
+ *       EPI_PROB    the last hidden map with the 1-wide output map folded in (the tile spans
+ *                   every column), for inference: logit = b_out + sum_n SiLU(acc + b)_n w_out[n],
+ *                   and its sigmoid;
+ *       EPI_HEAD    the same for training, on a cluster of 64-column tiles: the row's sigmoid
+ *                   cross-entropy, dlogit = (sigmoid - y) / rows, SiLU(z) transposed, and the
+ *                   gradient of the hidden map's pre-activation dz = dlogit w_out SiLU'(z) as
+ *                   BF16 rows and columns;
  *       EPI_BACK    dz_prev = acc * SiLU'(z_prev) (acc = dz W, the gradient reaching the
  *                   previous map's output) as BF16 rows and columns;
  *       EPI_F32     the FP32 accumulators themselves, column-major so that a warp's stores
@@ -50,7 +51,7 @@ constexpr int kBlockK = 64;           // K columns per stage: 128 bytes of BF16,
 constexpr int kThreads = 256;            // eight warps
 constexpr uint64_t kWaitNs = 2000000000ull;   // 2 s
 
-enum Epilogue { EPI_HIDDEN = 0, EPI_HEAD = 1, EPI_BACK = 2, EPI_F32 = 3 };
+enum Epilogue { EPI_HIDDEN = 0, EPI_HEAD = 1, EPI_BACK = 2, EPI_F32 = 3, EPI_PROB = 4 };
 
 struct EpiParams {
     int32_t M, N;                 // valid rows and columns of D
@@ -61,14 +62,14 @@ struct EpiParams {
     __nv_bfloat16 *rows;          // BF16 rows [M x ld_out]: h (HIDDEN) or dz (HEAD, BACK)
     __nv_bfloat16 *cols;          // BF16 columns [N x ld_t]: h^T (HIDDEN) or dz^T (HEAD, BACK)
     const float *z_prev;          // EPI_BACK: pre-activations of the previous map [M x ld_out]
-    const float *w_out;           // EPI_HEAD: output map weights [N] and bias [1]
+    const float *w_out;           // EPI_HEAD, EPI_PROB: output map weights [N] and bias [1]
     const float *b_out;
-    float *prob;                  // EPI_HEAD inference: sigmoid(logit) [M]
-    const float *y;               // EPI_HEAD training: targets [M]
-    float *dlogit;                // EPI_HEAD training: (sigmoid - y) / rows_total [M]
-    float *row_loss;              // EPI_HEAD training: per-row cross-entropy [M]
-    __nv_bfloat16 *h_cols;        // EPI_HEAD training: SiLU(z) transposed [N x ld_t]
-    float rows_total;             // EPI_HEAD training: the mean's denominator
+    float *prob;                  // EPI_PROB: sigmoid(logit) [M]
+    const float *y;               // EPI_HEAD: targets [M]
+    float *dlogit;                // EPI_HEAD: (sigmoid - y) / rows_total [M]
+    float *row_loss;              // EPI_HEAD: per-row cross-entropy [M]
+    __nv_bfloat16 *h_cols;        // EPI_HEAD: SiLU(z) transposed [N x ld_t]
+    float rows_total;             // EPI_HEAD: the mean's denominator
     float *out;                   // EPI_F32: D column-major, [splits][N][ld_out] (ld_out >= M)
     int32_t *err;
 };
@@ -156,6 +157,19 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
 __device__ __forceinline__ void mma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                  : "memory");
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
+/* The variable that *p is in this CTA's shared memory, in that of the cluster's CTA `rank`, = v. */
+__device__ __forceinline__ void cluster_store(float *p, uint32_t rank, float v) {
+    asm volatile(
+        "{\n\t.reg .b32 a;\n\t"
+        "mapa.shared::cluster.u32 a, %0, %1;\n\t"
+        "st.shared::cluster.f32 [a], %2;\n\t}\n"
+        ::"r"(smem_u32(p)), "r"(rank), "f"(v)
+        : "memory");
 }
 
 /* This thread's tensor-memory lane, 16 consecutive 32-bit columns from `taddr`. */
@@ -269,15 +283,28 @@ __device__ __forceinline__ void column_params(const float *p, int32_t nc, int32_
     }
 }
 
+/*
+ * EPI_HEAD: what bounds a training batch's head is the elementwise work, two special-function
+ * instructions per element and the stores.  A tile of all 256 columns left that to one CTA per 128
+ * rows, 128 columns per thread in two passes; a cluster of 64-column tiles spreads it over four
+ * SMs, 32 columns per thread held in registers (a training step of 645 -> 256 x 3 -> 1: 113.6 ->
+ * 97.3 us at 4,096 rows, 78.7 -> 62.4 at 256; two CTAs per SM, 128 registers, keep 65,536 rows where
+ * they were).  The logit's sum keeps EPI_PROB's order (columns
+ * 0-127 and 128-255 one after the other, then the two): it goes from half tile to half tile,
+ * through shared memory inside a CTA and through the neighbour's between two, 32 FMAs each.
+ *
+ * EPI_PROB keeps the 256-column tile: inference has one pass and no stores, its batches fill the
+ * chip with row tiles, and four tiles would read A four times (100,000 rows: 386 us for the
+ * network, 507 with the clusters; 2,000 rows: 40 and 39).
+ */
 template <int EPI, int BN>
 __device__ __forceinline__ void epilogue(const EpiParams &E, uint32_t tacc, int32_t row, int32_t c0, int32_t half,
-                                         int32_t split, float *s_logit, const float *pre) {
+                                         int32_t split, bool ok, float *s_logit, const float *pre) {
     constexpr int C = Shape<BN>::kCols;
-    const bool live = row < E.M;
+    const bool live = ok && row < E.M;
     const int32_t r = threadIdx.x & 127;   // row within the tile (quarter * 32 + lane)
-    if constexpr (EPI == EPI_HEAD) {
-        // pass 1: this half's share of the logit, SiLU(z) transposed (training)
-        float part = 0.0f;
+    if constexpr (EPI == EPI_PROB) {
+        float part = 0.0f;   // this half's share of the logit
 #pragma unroll 1
         for (int c = 0; c < C; c += 16) {
             float v[16], b[16], w[16];
@@ -288,42 +315,68 @@ __device__ __forceinline__ void epilogue(const EpiParams &E, uint32_t tacc, int3
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
                 const float z = v[j] + b[j];
-                v[j] = z * sigmoid_f(z);
-                part = fmaf(v[j], w[j], part);
+                part = fmaf(z * sigmoid_f(z), w[j], part);
             }
-            if (live && E.h_cols)
-#pragma unroll
-                for (int j = 0; j < 16; ++j)
-                    if (nc + j < E.N) E.h_cols[(int64_t)(nc + j) * E.ld_t + row] = __float2bfloat16(v[j]);
         }
         s_logit[half * kTileM + r] = part;
         __syncthreads();
-        const float logit = s_logit[r] + s_logit[kTileM + r] + E.b_out[0];
-        if (!E.y) {
-            if (live && half == 0) E.prob[row] = sigmoid_f(logit);
-            return;
-        }
-        float g = 0.0f;
-        if (live) {
-            const float t = E.y[row];
-            g = (sigmoid_f(logit) - t) / E.rows_total;
-            if (half == 0) {
-                E.row_loss[row] = fmaxf(logit, 0.0f) - logit * t + log1pf(__expf(-fabsf(logit)));
-                E.dlogit[row] = g;
+        if (live && half == 0) E.prob[row] = sigmoid_f(s_logit[r] + s_logit[kTileM + r] + E.b_out[0]);
+    } else if constexpr (EPI == EPI_HEAD) {
+        float h[C], grad[C];   // SiLU(z) and SiLU'(z)
+#pragma unroll
+        for (int c = 0; c < C; c += 16) {
+            float v[16];
+            tmem_ld16(tacc + c, v);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                const float z = v[j] + pre[c + j], s = sigmoid_f(z);
+                h[c + j] = z * s;
+                grad[c + j] = s * (1.0f + z * (1.0f - s));
             }
         }
-        // pass 2: the last hidden map's dz = dlogit w_out SiLU'(z)
-#pragma unroll 1
-        for (int c = 0; c < C; c += 16) {
-            float v[16], b[16], w[16];
-            tmem_ld16(tacc + c, v);
-            if (!live) continue;
-            const int32_t nc = c0 + c;
-            column_params(E.bias, nc, E.N, b);
-            column_params(E.w_out, nc, E.N, w);
+        if (live)
 #pragma unroll
-            for (int j = 0; j < 16; ++j) v[j] = g * w[j] * silu_grad(v[j] + b[j]);
-            store_rows_cols(E, row, nc, v);
+            for (int j = 0; j < C; ++j)
+                if (c0 + j < E.N) E.h_cols[(int64_t)(c0 + j) * E.ld_t + row] = __float2bfloat16(h[j]);
+        const uint32_t rank = blockIdx.y, tiles = gridDim.y;   // the cluster is the grid's column of tiles
+        float *s_link = s_logit + 2 * kTileM;
+        cluster_wait();   // every CTA of the cluster runs
+#pragma unroll
+        for (int link = 0; link < 4; ++link) {
+            if ((int)(rank & 1) * 2 + half == link) {
+                float part = link ? s_link[r] : 0.0f;
+#pragma unroll
+                for (int j = 0; j < C; ++j) part = fmaf(h[j], pre[C + j], part);
+                if (link == 3 || (link == 1 && rank + 1 == tiles)) {
+                    for (uint32_t q = 0; q < tiles; ++q) cluster_store(&s_logit[(rank / 2) * kTileM + r], q, part);
+                } else if (link == 1) {
+                    cluster_store(&s_link[r], rank + 1, part);
+                } else {
+                    s_link[r] = part;
+                }
+            }
+            if (link & 1) {
+                cluster_arrive();
+                cluster_wait();
+            } else {
+                __syncthreads();
+            }
+        }
+        const float logit = s_logit[r] + (tiles > 2 ? s_logit[kTileM + r] : 0.0f) + E.b_out[0];
+        if (!live) return;
+        const float t = E.y[row];
+        const float g = (sigmoid_f(logit) - t) / E.rows_total;
+        if (rank == 0 && half == 0) {   // one thread per row
+            E.row_loss[row] = fmaxf(logit, 0.0f) - logit * t + log1pf(__expf(-fabsf(logit)));
+            E.dlogit[row] = g;
+        }
+        // the last hidden map's dz = dlogit w_out SiLU'(z)
+#pragma unroll
+        for (int c = 0; c < C; c += 16) {
+            float v[16];
+#pragma unroll
+            for (int j = 0; j < 16; ++j) v[j] = g * pre[C + c + j] * grad[c + j];
+            if (c0 + c < E.N) store_rows_cols(E, row, c0 + c, v);
         }
     } else {
 #pragma unroll
@@ -365,12 +418,12 @@ __device__ __forceinline__ void epilogue(const EpiParams &E, uint32_t tacc, int3
  * Eight warps: warp 0 lane 0 issues the copies, warp 1 lane 0 the products, and all eight run
  * the epilogue (two per tensor-memory lane quarter, one column half each). */
 template <int EPI, int BN>
-__global__ void __launch_bounds__(kThreads, 1)
+__global__ void __launch_bounds__(kThreads, EPI == EPI_HEAD ? 2 : 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                      int32_t kb_total, int32_t kb_per_split, const EpiParams E) {
     using S = Shape<BN>;
     extern __shared__ unsigned char smem_raw[];
-    __shared__ float s_logit[2 * kTileM];
+    __shared__ float s_logit[EPI == EPI_HEAD ? 3 * kTileM : EPI == EPI_PROB ? 2 * kTileM : 1];
     __shared__ int failed;
     unsigned char *base = reinterpret_cast<unsigned char *>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
     uint64_t *full = reinterpret_cast<uint64_t *>(base + S::kStages * S::kStageBytes);
@@ -401,6 +454,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
+    if constexpr (EPI == EPI_HEAD) cluster_arrive();   // waited for in the epilogue
     const uint32_t tmem = *tmem_slot;
 
     if (nkb > 0 && warp == 0 && lane == 0) {
@@ -439,7 +493,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int quarter = warp & 3, half = warp >> 2;
     const int32_t row = m0 + quarter * 32 + lane, c0 = n0 + half * S::kCols;
     // operands of the epilogue that do not depend on the products, loaded while they run
-    float pre[EPI == EPI_BACK ? S::kCols : 1];
+    float pre[EPI == EPI_BACK ? S::kCols : EPI == EPI_HEAD ? 2 * S::kCols : 1];
+    if constexpr (EPI == EPI_HEAD) {
+#pragma unroll
+        for (int c = 0; c < S::kCols; c += 16) {
+            float b[16], w[16];
+            column_params(E.bias, c0 + c, E.N, b);
+            column_params(E.w_out, c0 + c, E.N, w);
+#pragma unroll
+            for (int j = 0; j < 16; ++j) {
+                pre[c + j] = b[j];
+                pre[S::kCols + c + j] = w[j];
+            }
+        }
+    }
     if constexpr (EPI == EPI_BACK) {
 #pragma unroll
         for (int c = 0; c < S::kCols; c += 16) {
@@ -457,12 +524,12 @@ __global__ void __launch_bounds__(kThreads, 1)
     }
     if (nkb <= 0 || !mbar_wait(done, 0)) atomicExch(&failed, 1);
     __syncthreads();
-    if (failed) {
-        if (threadIdx.x == 0) atomicMax(E.err, (int32_t)MIND_ETIMEOUT);
-    } else {
+    const bool ok = !failed;
+    if (!ok && threadIdx.x == 0) atomicMax(E.err, (int32_t)MIND_ETIMEOUT);
+    if (ok || EPI == EPI_HEAD) {   // a head tile's cluster waits for it: it stores nothing, but takes part
         tc_fence_after();
         const uint32_t tacc = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * S::kCols);
-        epilogue<EPI, BN>(E, tacc, row, c0, half, split, s_logit, pre);
+        epilogue<EPI, BN>(E, tacc, row, c0, half, split, ok, s_logit, pre);
     }
     tc_fence_before();
     __syncthreads();

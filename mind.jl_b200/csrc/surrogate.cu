@@ -8,8 +8,8 @@
  * tcgen05 kernels (mlp_umma.cuh) whose epilogues carry the elementwise work:
  *
  *   forward   map l < last hidden:  z_l = h_l W_l^T + b_l, h_{l+1} = SiLU(z_l)      EPI_HIDDEN
- *             last hidden map + output map: logit, sigmoid (inference), or the
- *             cross-entropy, dlogit and dz of the last hidden map (training)          EPI_HEAD
+ *             last hidden map + output map: logit and sigmoid (inference),            EPI_PROB
+ *             or cross-entropy, dlogit and dz of the last hidden map (training)       EPI_HEAD
  *   backward  dW_l = dz_l^T h_l (rows split into K slices, summed in a fixed order)   EPI_F32
  *             dz_{l-1} = (dz_l W_l) * SiLU'(z_{l-1})                                  EPI_BACK
  *
@@ -19,7 +19,7 @@
  * ones).  The products' operands are K-major everywhere, so every activation and gradient
  * that a weight gradient needs is also written transposed (rows of the batch contiguous).
  * Parameter layout: for each linear map l, W_l [out x in] row-major, then b_l [out], maps in
- * order.  hidden must be a multiple of 16 and at most 256 (one tile spans a hidden layer).
+ * order.  hidden must be a multiple of 16 and at most 256 (one tile, or a cluster's, spans a hidden layer).
  */
 #include <cuda.h>
 #include <cudaTypedefs.h>
@@ -314,7 +314,23 @@ int product(MindMlp *m, const __nv_bfloat16 *A, int64_t lda, const __nv_bfloat16
     E.N = N;
     E.err = m->err;
     const dim3 g((M + mlp::kTileM - 1) / mlp::kTileM, (N + BN - 1) / BN, splits);
-    mlp::umma_gemm_kernel<EPI, BN><<<g, mlp::kThreads, S::kSmemBytes, s>>>(ma, mb, kb_total, per, E);
+    if constexpr (EPI == mlp::EPI_HEAD) {   // the tiles of a row form a cluster (at most 256 / BN CTAs)
+        cudaLaunchAttribute cluster{};
+        cluster.id = cudaLaunchAttributeClusterDimension;
+        cluster.val.clusterDim.x = 1;
+        cluster.val.clusterDim.y = g.y;
+        cluster.val.clusterDim.z = 1;
+        cudaLaunchConfig_t config{};
+        config.gridDim = g;
+        config.blockDim = dim3(mlp::kThreads);
+        config.dynamicSmemBytes = S::kSmemBytes;
+        config.stream = s;
+        config.attrs = &cluster;
+        config.numAttrs = 1;
+        MLP_CUDA(m, cudaLaunchKernelEx(&config, mlp::umma_gemm_kernel<EPI, BN>, ma, mb, kb_total, per, E));
+    } else {
+        mlp::umma_gemm_kernel<EPI, BN><<<g, mlp::kThreads, S::kSmemBytes, s>>>(ma, mb, kb_total, per, E);
+    }
     MLP_CUDA(m, cudaGetLastError());
     return MIND_OK;
 }
@@ -327,7 +343,9 @@ int prepare_products(MindMlp *m) {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::Shape<64>::kSmemBytes));
     MLP_CUDA(m, cudaFuncSetAttribute(mlp::umma_gemm_kernel<mlp::EPI_F32, 64>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::Shape<64>::kSmemBytes));
-    MLP_CUDA(m, cudaFuncSetAttribute(mlp::umma_gemm_kernel<mlp::EPI_HEAD, 256>,
+    MLP_CUDA(m, cudaFuncSetAttribute(mlp::umma_gemm_kernel<mlp::EPI_HEAD, 64>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::Shape<64>::kSmemBytes));
+    MLP_CUDA(m, cudaFuncSetAttribute(mlp::umma_gemm_kernel<mlp::EPI_PROB, 256>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::Shape<256>::kSmemBytes));
     return MIND_OK;
 }
@@ -438,10 +456,11 @@ int forward(MindMlp *m, int64_t rows, bool train, cudaStream_t s, float *prob = 
                 E.rows = m->dzr[0];
                 E.cols = m->dzc[0];
                 E.rows_total = (float)rows;
+                MLP_TRY((product<mlp::EPI_HEAD, 64>(m, A, lda, W, K, R, H, K, 1, E, s)));
             } else {
                 E.prob = prob ? prob : m->prob;
+                MLP_TRY((product<mlp::EPI_PROB, 256>(m, A, lda, W, K, R, H, K, 1, E, s)));
             }
-            MLP_TRY((product<mlp::EPI_HEAD, 256>(m, A, lda, W, K, R, H, K, 1, E, s)));
         }
     }
     return MIND_OK;

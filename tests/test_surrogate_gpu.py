@@ -256,3 +256,22 @@ def test_gradients_on_side_streams_repeat_bit_for_bit(layers, hidden, rows):
         runs.append((losses, net.params))
         net.close()
     assert np.array_equal(runs[0][0], runs[1][0]) and np.array_equal(runs[0][1], runs[1][1])
+
+
+@pytest.mark.parametrize("hidden", [16, 64, 80, 128, 144, 192, 208, 256])
+@pytest.mark.parametrize("layers,rows", [(1, 129), (3, 300)])
+def test_head_clusters_of_every_width(hidden, layers, rows):
+    """The head's 64-column tiles, one to four to a cluster, the last one whole or partial: the
+    gradient and the probabilities against the oracle, within the BF16 bounds of the tests above."""
+    rng = np.random.default_rng(hidden)
+    net = surrogate.Mlp(n_in=37, hidden=hidden, layers=layers, seed=6)
+    dims = [37] + [hidden] * layers + [1]
+    x = rng.normal(0.0, 1.0, (rows, 37)).astype(np.float32)
+    y = (rng.uniform(size=rows) < 0.3).astype(np.float32)
+    params = net.params.astype(np.float64)
+    want_loss, want = oracle_mlp.loss_and_gradients(params, dims, x, y)
+    got, loss = net.gradients(x, y)
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < 5e-2
+    assert abs(loss - want_loss) < 1e-2 * want_loss
+    np.testing.assert_allclose(net.predict(x), oracle_mlp.predict(params, dims, x), atol=1e-2)
+    net.close()
