@@ -36,6 +36,7 @@
 
 #include "../../include/mindgpu.h"
 #include "mlp_umma.cuh"
+#include "upload.hpp"
 
 struct MindMlp {
     std::vector<int32_t> dims;       // n_in, hidden..., 1
@@ -71,6 +72,7 @@ struct MindMlp {
     cudaEvent_t t0 = nullptr, t1 = nullptr;
     float *data_x = nullptr, *data_y = nullptr;  // training set (FP32 on the device)
     int64_t data_n = 0, data_cap = 0;
+    Uploader uploader;               // input rows and training sets from pageable memory
     // The backward pass beside the chain of dz products (see backward()): weight gradients on
     // side[0], sums over rows on side[1].
     cudaStream_t side[2] = {nullptr, nullptr};
@@ -397,6 +399,7 @@ int reserve(MindMlp *m, int64_t rows) {
     }
     MLP_CUDA(m, cudaMalloc(&m->x, cap * m->ld0 * sizeof(__nv_bfloat16)));
     MLP_CUDA(m, cudaMalloc(&m->xin, cap * m->dims[0] * sizeof(float)));
+    m->uploader.reserve(cap * m->dims[0] * sizeof(float));
     MLP_CUDA(m, cudaMalloc(&m->xt, (int64_t)m->ld0 * capT * sizeof(__nv_bfloat16)));
     MLP_CUDA(m, cudaMalloc(&m->ht_last, H * capT * sizeof(__nv_bfloat16)));
     for (int k = 0; k < 2; ++k) {
@@ -549,7 +552,7 @@ int backward(MindMlp *m, int64_t rows, cudaStream_t s) {
 int upload_rows(MindMlp *m, const float *x, int64_t n) {
     (void)cudaGetLastError();
     MLP_TRY(reserve(m, n));
-    MLP_CUDA(m, cudaMemcpyAsync(m->xin, x, n * m->dims[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    MLP_CUDA(m, m->uploader.copy(m->xin, x, n * m->dims[0] * sizeof(float), m->stream));
     MLP_CUDA(m, cudaEventRecord(m->t0, m->stream));
     to_bf16_rows_kernel<<<row_grid(n, m->ld0), kT, 0, m->stream>>>(m->xin, m->x, n, m->dims[0], m->ld0);
     return MIND_OK;
@@ -653,6 +656,7 @@ int mind_mlp_destroy(MindMlp *m) {
     if (!m) return MIND_OK;
     for (cudaStream_t s : {m->stream, m->side[0], m->side[1]})
         if (s) cudaStreamSynchronize(s);
+    m->uploader.release();
     free_activations(m);
     for (void *p : {(void *)m->master, (void *)m->grad, (void *)m->m1, (void *)m->m2, (void *)m->wbf, (void *)m->w0,
                     (void *)m->wt, (void *)m->loss, (void *)m->loss_hist, (void *)m->data_x, (void *)m->data_y,
@@ -755,10 +759,11 @@ int mind_mlp_set_data(MindMlp *m, const float *x, const float *y, int64_t n) {
         cudaFree(m->data_y);
         m->data_x = m->data_y = nullptr;
         MLP_CUDA(m, cudaMalloc(&m->data_x, n * m->dims[0] * sizeof(float)));
+        m->uploader.reserve(n * m->dims[0] * sizeof(float));
         MLP_CUDA(m, cudaMalloc(&m->data_y, n * sizeof(float)));
         m->data_cap = n;
     }
-    MLP_CUDA(m, cudaMemcpyAsync(m->data_x, x, n * m->dims[0] * sizeof(float), cudaMemcpyHostToDevice, m->stream));
+    MLP_CUDA(m, m->uploader.copy(m->data_x, x, n * m->dims[0] * sizeof(float), m->stream));
     MLP_CUDA(m, cudaMemcpyAsync(m->data_y, y, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MLP_CUDA(m, cudaStreamSynchronize(m->stream));
     m->data_n = n;

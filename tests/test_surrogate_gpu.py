@@ -275,3 +275,24 @@ def test_head_clusters_of_every_width(hidden, layers, rows):
     assert abs(loss - want_loss) < 1e-2 * want_loss
     np.testing.assert_allclose(net.predict(x), oracle_mlp.predict(params, dims, x), atol=1e-2)
     net.close()
+
+
+@pytest.mark.parametrize("rows", [1623, 1626, 1627, 20011])
+def test_staged_uploads_bring_every_byte(rows):
+    """Inputs around the size where a copy from pageable memory is staged (4 MB), ending inside a
+    512 KB piece: rows predicted at once equal the same rows in small calls, from views of any
+    alignment and from pinned memory, and again with other rows in the same buffers."""
+    import torch
+
+    rng = np.random.default_rng(rows)
+    net = surrogate.Mlp(seed=9)
+    flat = rng.normal(0.0, 1.0, rows * surrogate.N_FEATURES + 1).astype(np.float32)
+    for x in (flat[1:].reshape(rows, -1), flat[:-1].reshape(rows, -1)):
+        whole = net.predict(x)
+        small = surrogate.Mlp(seed=9)
+        parts = np.concatenate([small.predict(x[k:k + 128]) for k in range(0, rows, 128)])
+        small.close()
+        assert np.array_equal(whole, parts)
+        pinned = torch.from_numpy(x.copy()).pin_memory().numpy()
+        assert np.array_equal(net.predict(pinned), whole)
+    net.close()
