@@ -663,7 +663,7 @@ __device__ __forceinline__ void hines(double2 *sdr, const double *sa, double *sx
  *
  * The Hines solve runs level by level, one path per thread (a chain, or on cells the plan
  * gave paths a chain and the child chains it continues); along a chain only subtract ->
- * divide -> multiply stays on the dependency chain, the next node's operands being loaded
+ * quotient -> multiply stays on the dependency chain, the next node's operands being loaded
  * ahead.  PATHS false compiles the one-chain-per-thread loops only, for launches whose
  * cells all have the chain schedule.
  */
