@@ -759,7 +759,10 @@ int mind_mlp_set_data(MindMlp *m, const float *x, const float *y, int64_t n) {
         cudaFree(m->data_y);
         m->data_x = m->data_y = nullptr;
         MLP_CUDA(m, cudaMalloc(&m->data_x, n * m->dims[0] * sizeof(float)));
-        m->uploader.reserve(n * m->dims[0] * sizeof(float));
+        // a set is usually copied once: making the buffers (about 2 ms) is repaid from 64 MB on; where
+        // predict made them, smaller sets use them too
+        const size_t bytes = n * m->dims[0] * sizeof(float);
+        if (bytes >= ((size_t)64 << 20)) m->uploader.reserve(bytes);
         MLP_CUDA(m, cudaMalloc(&m->data_y, n * sizeof(float)));
         m->data_cap = n;
     }
