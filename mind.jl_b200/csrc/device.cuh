@@ -83,7 +83,8 @@ struct DevGroup {
     float *s[4];              // FP32 decay factors of the synapses (mixed mode)
     // mechanisms emitted from MOD files (kind MIND_MECH_GENERATED + gen): their fields as
     // ncols columns of `cols` (column k of row r at cols[k * rows + r]), then one column of
-    // current scale (area * 0.01 for density mechanisms, 1 for point processes)
+    // current scale (area * 0.01 for density mechanisms, 1 for point processes) and two that keep
+    // a row's terms of a step for its second solve
     double *cols;
     int32_t ncols;
     int32_t gen;              // index into kGenMechanisms, -1 for the hand-written kinds

@@ -1017,19 +1017,34 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     }
                 } else if (GEN && GG.gen >= 0) {
                     // emitted from a MOD file: BREAKPOINT probed at v + 0.001 and at v
-                    // (src/runtime/cuda/micro.jl:427-500); the second call's writes persist
+                    // (src/runtime/cuda/micro.jl:427-500); the second call's writes persist.  They may
+                    // feed a later call (a counter, a filter), so a step that is assembled again takes
+                    // the row's two terms from where the first pass kept them.
                     const int32_t *pn = GG.node + G.r0;
                     const double *pscale = GG.cols + (int64_t)GG.ncols * GG.rows + G.r0;
+                    double *kept_y = GG.cols + (int64_t)(GG.ncols + 1) * GG.rows + G.r0, *kept_x = kept_y + GG.rows;
                     for (int32_t r = lo; r < hi; ++r) {
                         const int32_t node = (int32_t)(__ldg(pn + r) - nb);
-                        const double vv = sv[node];
-                        MindGenRow row{GG.cols, GG.rows, (int64_t)G.r0 + r, vv + 0.001, tc, P.dt, P.celsius};
-                        const double shifted = gen_current(GG.gen, row);
-                        row.v = vv;
-                        const double value = gen_current(GG.gen, row);
-                        const double scale = pscale[r];
-                        sdr[node].y = sdr[node].y - scale * value;
-                        sdr[node].x = sdr[node].x + milli_quotient<MIXED>(scale * (shifted - value));
+                        double ty, tx;
+                        if (!MIXED && exact) {
+                            ty = kept_y[r];
+                            tx = kept_x[r];
+                        } else {
+                            const double vv = sv[node];
+                            MindGenRow row{GG.cols, GG.rows, (int64_t)G.r0 + r, vv + 0.001, tc, P.dt, P.celsius};
+                            const double shifted = gen_current(GG.gen, row);
+                            row.v = vv;
+                            const double value = gen_current(GG.gen, row);
+                            const double scale = pscale[r];
+                            ty = scale * value;
+                            tx = milli_quotient<MIXED>(scale * (shifted - value));
+                            if (!MIXED) {
+                                kept_y[r] = ty;
+                                kept_x[r] = tx;
+                            }
+                        }
+                        sdr[node].y = sdr[node].y - ty;
+                        sdr[node].x = sdr[node].x + tx;
                     }
                 } else if (G.kind == MIND_MECH_HH) {
                     for (int32_t r = lo; r < hi; ++r) {

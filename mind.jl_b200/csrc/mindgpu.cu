@@ -810,7 +810,8 @@ int create(const MindLayout *L, MindHandle *h) {
         h->has_generated |= generated;
         h->gen_runtime |= generated && m.kind - MIND_MECH_GENERATED >= kGeneratedCount;
         G.ncols = generated ? gen_cols : 0;
-        G.cols = generated ? h->alloc<double>((size_t)(gen_cols + 1) * (size_t)std::max(rows, 1)) : nullptr;
+        // the fields, the scale, and the two terms of a row that a repeated step takes again
+        G.cols = generated ? h->alloc<double>((size_t)(gen_cols + 3) * (size_t)std::max(rows, 1)) : nullptr;
         h->group_init.push_back(std::move(init));
     }
 
