@@ -262,12 +262,13 @@ struct Params {
     const int32_t *ns_source;      // per NetStim row: 0-based source or -1
     // recording
     const int32_t *rec_off;        // [ncells+1]
-    // per record of the cell: rec_ptr non-null reads that HBM value (a constant parameter);
+    // per record of the cell: rec_ptr non-null reads that HBM value (a parameter, an emitted field);
     // else rec_node >= 0 is a local node's v and rec_node < 0 a staged field,
     // -1 - rec_node = group << 24 | staged slot << 20 | row within the cell's rows
     const int32_t *rec_node;
     const double *const *rec_ptr;
     const int32_t *rec_col;
+    int32_t rec_state;             // some record is of state that a step advances, in shared memory or HBM
     double *trace;
     // cells the surrogate stands in for (null: none) and their drive ring [kSurrogateRing][ncells][32]
     const uint8_t *cell_mode;

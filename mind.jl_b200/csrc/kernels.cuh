@@ -849,16 +849,12 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
         sw[k] = P.groups[g].kind == MIND_MECH_EXP2SYN ? w * P.groups[g].f[E2_FACTOR][drow] : w;
         e.point = (g << 24) | (drow - sg[g].r0);
     }
-    const int32_t rec_lo = P.nrec ? P.rec_off[c] : 0, rec_hi = P.nrec ? P.rec_off[c + 1] : 0;
-    // Mechanism state is recorded by another thread than the one that advances it, so a cell
-    // with such a record has a barrier in between; voltages have one behind the solve.
-    bool state_recorded = false;
-    for (int32_t k = rec_lo + tid; k < rec_hi; k += T) state_recorded |= P.rec_ptr[k] || P.rec_node[k] < 0;
-    state_recorded = __syncthreads_or(state_recorded);
+    __syncthreads();
 
     const double q10 = mind_pow(3.0, (P.celsius - 6.3) / 10.0);
     const float q10f = (float)q10;
     // The thread's first recorded quantity stays in registers for the window.
+    const int32_t rec_lo = P.nrec ? P.rec_off[c] : 0, rec_hi = P.nrec ? P.rec_off[c + 1] : 0;
     auto record = [&](int32_t code, const double *gp) -> double {
         if (gp) return *gp;
         if (code >= 0) return sv[code];
@@ -1225,8 +1221,9 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     break;
             }
         }
-        // 9. Record the completed boundary.
-        if (state_recorded) __syncthreads();
+        // 9. Record the completed boundary.  Mechanism state is recorded by another thread than the
+        //    one that has just advanced it; voltages have a barrier behind the solve.
+        if (P.rec_state) __syncthreads();
         if (records) {
             const int64_t sample = step + 1 - P.run_start;
             P.trace[sample * P.nrec + rec_col] = record(rec_code, rec_ptr);

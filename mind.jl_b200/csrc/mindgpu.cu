@@ -167,6 +167,7 @@ struct MindHandle {
     size_t trace_capacity = 0;
     size_t rec_capacity = 0, rec_off_cap = 0, rec_col_cap = 0, rec_ptr_cap = 0, rec_initial_cap = 0;
     std::vector<MindRecord> rec_last;             // the record set whose tables are on the device
+    bool rec_last_state = false;                  // Params::rec_state of that set
     struct Bin {
         int32_t first, count;
         size_t smem_bytes;
@@ -1176,6 +1177,7 @@ int check_device_error(MindHandle *h) {
 struct RecordTarget {
     int32_t cell = -1;
     int32_t code = 0;
+    bool state = false;   // a step's state advance may write it
     const double *ptr = nullptr;
     const double *initial = nullptr;
 };
@@ -1219,8 +1221,9 @@ int resolve_record(MindHandle *h, const MindRecord &rec, RecordTarget &out) {
         return fail(h, MIND_EARG, "a recorded state row lies beyond 2^20 rows of its cell");
     } else {
         out.code = 0;
-        out.ptr = out.initial;   // a parameter: constant through the run
+        out.ptr = out.initial;   // a parameter, or an emitted mechanism's field
     }
+    out.state = ss >= 0 || generated_kind(kind);
     return MIND_OK;
 }
 
@@ -1229,6 +1232,7 @@ int resolve_record(MindHandle *h, const MindRecord &rec, RecordTarget &out) {
 struct RecordTables {
     std::vector<int32_t> off, code, col;
     std::vector<const double *> ptr, initial;
+    bool state = false;   // Params::rec_state
 };
 
 int build_records(MindHandle *h, const MindRecord *records, int32_t nrec, RecordTables &t) {
@@ -1240,6 +1244,7 @@ int build_records(MindHandle *h, const MindRecord *records, int32_t nrec, Record
         if (status) return status;
         if (target.cell < 0) return fail(h, MIND_EARG, "NetStim fields are read with mind_read_value, not recorded");
         t.initial[k] = target.initial;
+        t.state |= target.state;
         by_cell[target.cell].push_back({target, k});
     }
     t.off.assign(1, 0);
@@ -1297,11 +1302,13 @@ int set_records(MindHandle *h, const MindRecord *records, int32_t nrec, int64_t 
         }
         // pageable sources: the copies above have consumed the host tables when they return
         h->rec_last.assign(records, records + nrec);
+        h->rec_last_state = t.state;
     }
     P.rec_off = h->rec_off_dev;
     P.rec_node = h->rec_node_dev;
     P.rec_ptr = h->rec_ptr_dev;
     P.rec_col = h->rec_col_dev;
+    P.rec_state = h->rec_last_state ? 1 : 0;
     P.nrec = nrec;
     size_t need = (size_t)samples * (size_t)std::max(nrec, 1);
     if (nrec > 0 && need > h->trace_capacity) {
@@ -2463,6 +2470,7 @@ int mind_run_noalloc(MindHandle *h, int64_t steps, const MindRecord *records, in
         P.rec_node = own.rec_node;
         P.rec_ptr = own.rec_ptr;
         P.rec_col = own.rec_col;
+        P.rec_state = own.rec_state;
         P.nrec = own.nrec;
         P.trace = own.trace;
         P.trace_samples = own.trace_samples;
@@ -2472,6 +2480,7 @@ int mind_run_noalloc(MindHandle *h, int64_t steps, const MindRecord *records, in
     P.rec_node = d_node;
     P.rec_ptr = d_ptr;
     P.rec_col = d_col;
+    P.rec_state = t.state ? 1 : 0;
     P.nrec = n_records;
     P.trace = d_trace;
     P.trace_samples = steps + 1;
