@@ -18,7 +18,8 @@ OUT_DIR = os.path.join(PACKAGE, "lib")
 OUTPUT = os.path.join(OUT_DIR, "libmindgpu.so")
 SOURCES = [os.path.join(HERE, "mindgpu.cu"), os.path.join(HERE, "surrogate.cu"), os.path.join(HERE, "planner.cpp")]
 DEPENDS = SOURCES + [os.path.join(HERE, f) for f in ("device.cuh", "kernels.cuh", "macro.cuh", "mind_math.h",
-                                                     "gen_runtime.cuh", "generated_mechanisms.cuh", "mlp_umma.cuh", "upload.hpp")] + [
+                                                     "gen_runtime.cuh", "generated_mechanisms.cuh", "mlp_umma.cuh", "quotient.cuh",
+                                                     "upload.hpp")] + [
     os.path.join(os.path.dirname(PACKAGE), "include", "mindgpu.h")]
 
 NVCC_FLAGS = [

@@ -203,7 +203,7 @@ struct Params {
     const int32_t *path_off;     // [ncells+1] into path_chain
     const int32_t *path_chain;   // per cell: npaths+1 local chain starts; only the sentinel for a
                                  // cell on the chain schedule (its paths are its chains)
-    int32_t axial_ok;          // every axial conductance is 0 or in [2^-480, 2^480)
+    uint8_t *divide;             // per cell: its last step lay outside the quotients' range (FP64 mode)
     DevGroup groups[kMaxGroups];
     // per cell, placed group and owner slot: first row (relative to the cell's first row of the group)
     // of the owner's rows; owner slot t holds the local nodes i with

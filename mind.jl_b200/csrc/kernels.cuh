@@ -18,6 +18,7 @@
 #include <type_traits>
 
 #include "device.cuh"
+#include "quotient.cuh"
 
 namespace mind {
 
@@ -490,59 +491,6 @@ __device__ __forceinline__ void apply_event(const StagedGroup &G, int32_t row, d
 
 __device__ __forceinline__ bool bad_pivot(double D) { return (D == 0.0) | !isfinite(D); }
 
-/* Where the quotients below are exact: magnitudes in [2^-480, 2^480), where nothing can overflow
- * or lose bits to underflow, and for the divisor no significand that starts with twenty ones (of
- * which the all-ones one is an exception of the method).  A quotient in [2^-400, 2^400) of a
- * divisor in range came from a numerator in range, and a zero from a zero or from an underflow
- * that the division shares. */
-__device__ __forceinline__ bool in_binades(double x, uint32_t low, uint32_t high) {
-    return ((uint32_t)__double2hiint(x) & 0x7FFFFFFFu) - (low << 20) < (high - low) << 20;
-}
-__device__ __forceinline__ bool good_divisor(double D) {
-    return in_binades(D, 1023u - 480u, 1023u + 480u) && (((uint32_t)__double2hiint(D) + 1u) & 0xFFFFFu) != 0u;
-}
-__device__ __forceinline__ bool good_quotient(double x) { return x == 0.0 || in_binades(x, 1023u - 400u, 1023u + 400u); }
-
-/*
- * IEEE quotients of the FP64 solve without the division's branches (a dependent division
- * measured 127 cycles on a B200, an FP64 fma 8.6, rcp.approx.ftz.f64 17.7), after
- * P. W. Markstein, "Computation of elementary functions on the IBM RISC System/6000
- * processor", IBM J. Res. Dev. 34(1), 1990, and J.-M. Muller et al., Handbook of
- * Floating-Point Arithmetic, chapter on FMA-based division:
- *   - two Newton steps on a seed good to 2^-19 leave y2 within one unit in the last place of
- *     1/D, and a third, y3 = y2 + y2 (1 - D y2) with the residual exact in one FMA, rounds to
- *     the nearest double of 1/D;
- *   - q1 = q0 + (n - D q0) y is within one unit in the last place of n/D, its residual
- *     r1 = n - D q1 is exact, and q1 + r1 y3 rounds to the IEEE quotient.
- */
-__device__ __forceinline__ double reciprocal_seed(double D) {
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(D));
-    return y;
-}
-__device__ __forceinline__ double reciprocal(double D) {
-    double y = reciprocal_seed(D);
-    y = fma(y, fma(-D, y, 1.0), y);
-    y = fma(y, fma(-D, y, 1.0), y);
-    return fma(y, fma(-D, y, 1.0), y);
-}
-/* n / D from D's reciprocal. */
-__device__ __forceinline__ double quotient(double n, double D, double y) {
-    const double q0 = n * y;
-    const double q1 = fma(fma(-D, q0, n), y, q0);
-    return fma(fma(-D, q1, n), y, q1);
-}
-/* a / D with D just known: the quotient starts from the reciprocal's first iterate. */
-__device__ __forceinline__ double pivot_quotient(double a, double D) {
-    const double y0 = reciprocal_seed(D);
-    const double y1 = fma(y0, fma(-D, y0, 1.0), y0);
-    const double q0 = a * y1;
-    const double y2 = fma(y1, fma(-D, y1, 1.0), y1);
-    const double q1 = fma(fma(-D, q0, a), y2, q0);
-    const double y3 = fma(y2, fma(-D, y2, 1.0), y2);
-    return fma(fma(-D, q1, a), y3, q1);
-}
-
 /*
  * Hines solve of one resident cell, level by level, one path per thread: a path is one chain, or a
  * chain and the child chains it continues when the cell's plan merged them; a path's chains
@@ -553,8 +501,8 @@ __device__ __forceinline__ double pivot_quotient(double a, double D) {
  *
  * FP64 mode: the reference's operations in the canonical order (gather-form elimination, f = a/D,
  * back-substitution (R + a x_p)/D), the quotients by pivot_quotient and quotient; the caller
- * checks afterwards that every one was in their range, and repeats the solve with EXACT,
- * which divides, where one was not.  Mixed mode: f = a y and R y in place of D and R with
+ * checks afterwards that every one was in their range (quotient.cuh), and repeats the solve with
+ * EXACT, which divides, where one was not.  Mixed mode: f = a y and R y in place of D and R with
  * y = approx_reciprocal(D), so the back-substitution is one FMA per node, x = f x_p + R y.
  *
  * What bounds it is the instructions of a node: the few lanes that hold the level's longest
@@ -671,6 +619,14 @@ template <bool MIXED, int NT, bool GLOBAL_IMAGE = false, bool GEN = false, bool 
 __device__ __forceinline__ void window_body(const Params &P, const int32_t *cells, int64_t n0, int32_t W) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ StagedGroup sg[kMaxGroups];
+    // FP64: how the step is solved.  A step outside the quotients' range is assembled and solved
+    // again with divisions, and the steps after it divide at once for as long as their own values
+    // stay outside, in later windows too (P.divide): a long cable at rest, in which the change from
+    // a stimulus fades to nothing along the way, stays there for all its run (400 compartments of
+    // 50 um x 0.5 um, 64 cells: 74 us per step with divisions only, 113 with every step solved
+    // twice, 73 so).  In shared memory, at a load per step; in registers it cost up to 3%.
+    constexpr int kDivide = 1, kAgain = 2, kFarAxial = 4;
+    __shared__ int how;
     const int32_t c = cells[blockIdx.x];
     const int32_t tid = threadIdx.x;
     constexpr int32_t T = NT;            // threads of this launch
@@ -784,9 +740,12 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
             }
         return;
     }
+    bool far_axial = false;   // an axial term beyond the range of the quotients by FMA
     for (int32_t i = tid; i < n; i += T) {
         sv[i] = P.v[nb + i];
-        sa[i] = P.a[nb + i];
+        const double a = P.a[nb + i];
+        sa[i] = a;
+        if (!MIXED) far_axial |= !good_axial(a);
     }
     for (int32_t k = tid; k < nch; k += T) {
         ctop[k] = P.chain_top[cb + k];
@@ -799,7 +758,8 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     for (int32_t k = tid; k <= nlev; k += T) lvp[k] = P.level_path[lv0 + k];
     for (int32_t k = tid; k <= npath; k += T) pch[k] = P.path_chain[pb + k];
     for (int32_t k = tid; k < P.nparts * (O + 1); k += T) spart[k] = (Index)P.part[(int64_t)c * P.nparts * (O + 1) + k];
-    __syncthreads();
+    far_axial = __syncthreads_or(far_axial);
+    if (!MIXED && tid == 0) how = far_axial ? kDivide | kFarAxial : P.divide[c] ? kDivide : 0;
     for (int32_t k = tid; k < nch; k += T)
         for (int32_t i = ctop[k]; i < ctop[k] + clen[k]; ++i) chain_of[i] = (int16_t)k;
     for (int32_t g = 0; g < P.ngroups; ++g) {
@@ -867,7 +827,6 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     const int32_t rec_col = records ? P.rec_col[rec_lo + tid] : 0;
     int32_t cursor = 0;
     bool singular = false;
-    bool exact = false;   // solve this step with divisions
 
     for (int32_t s = 0; s < W; ++s) {
         const int64_t step = n0 + s;
@@ -947,6 +906,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
         bool unsynced = false;   // rows of a group that was not halved may be in flight
         if (kShared) __syncthreads();
         const double tc = t + 0.5 * P.dt;
+        const bool again = GEN && !MIXED && (how & kAgain);   // the step's second assembly
         for (int32_t g = 0; g < P.ngroups; ++g) {
             const DevGroup &GG = P.groups[g];
             const StagedGroup G = sg[g];
@@ -1022,7 +982,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                     for (int32_t r = lo; r < hi; ++r) {
                         const int32_t node = (int32_t)(__ldg(pn + r) - nb);
                         double ty, tx;
-                        if (!MIXED && exact) {
+                        if (again) {
                             ty = kept_y[r];
                             tx = kept_x[r];
                         } else {
@@ -1126,7 +1086,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
         // 6-7. Hines elimination level by level, each chain bottom to top into its parent, then
         //      back-substitution root chain first, and the voltage update.
         const int32_t *paths = PATHS && npath ? pch : nullptr;
-        if (exact)
+        if (!MIXED && (how & kDivide))
             hines<MIXED, true, NT>(sdr, sa, sxd, sxr, ctop, clen, cpar, ckoff, ckids, lvp, paths, nlev, singular);
         else
             hines<MIXED, false, NT>(sdr, sa, sxd, sxr, ctop, clen, cpar, ckoff, ckids, lvp, paths, nlev, singular);
@@ -1137,13 +1097,22 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
                 sv[i] = sv[i] + P.vscale * fx.y;
             }
         } else {
-            bool good = P.axial_ok != 0;
-            for (int32_t i = tid; i < n; i += T) good &= good_divisor(sdr[i].x) && good_quotient(sdr[i].y);
-            if (__syncthreads_or(!good && !exact)) {   // assemble again, and divide
-                exact = true;
-                goto assemble;
+            // by the high words alone first: one step in about a million node-steps, and cables at
+            // rest, go on to the whole check
+            bool good = true;
+            for (int32_t i = tid; i < n; i += T) good &= surely_good(sdr[i].x, sdr[i].y);
+            if (__syncthreads_or(!good) || how) {
+                const int now = how;
+                good = !(now & kFarAxial);
+                for (int32_t i = tid; i < n; i += T) good &= good_divisor(sdr[i].x) && good_quotient(sdr[i].y, sdr[i].x);
+                const bool outside = __syncthreads_or(!good);
+                const bool repeat = outside && !(now & kDivide);
+                if (tid == 0) how = outside ? (now & kFarAxial) | kDivide | (repeat ? kAgain : 0) : 0;
+                if (repeat) {
+                    __syncthreads();
+                    goto assemble;
+                }
             }
-            exact = false;
             for (int32_t i = tid; i < n; i += T) sv[i] = sv[i] + P.vscale * sdr[i].y;
         }
         __syncthreads();
@@ -1237,6 +1206,7 @@ __device__ __forceinline__ void window_body(const Params &P, const int32_t *cell
     // ---- write back, with validate_device_state!'s finite check (src/runtime/utils/step.jl:168-197)
     //      of the written voltage and state; an earlier error code is kept ----
     if (my_det >= 0) P.above[my_src] = my_above ? 1 : 0;
+    if (!MIXED && tid == 0) P.divide[c] = how & kDivide;
     bool finite = true;
     for (int32_t i = tid; i < n; i += T) {
         P.v[nb + i] = sv[i];

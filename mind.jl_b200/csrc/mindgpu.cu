@@ -937,11 +937,7 @@ int create(const MindLayout *L, MindHandle *h) {
     P.level_path = h->upload(level_path);
     P.path_off = h->upload(path_off);
     P.path_chain = h->upload(path_chain);
-    P.axial_ok = 1;
-    for (double x : a) {
-        const double m = std::fabs(x);
-        if (m != 0.0 && !(m >= 0x1p-480 && m < 0x1p480)) P.axial_ok = 0;
-    }
+    P.divide = h->alloc<uint8_t>(ncells);   // cleared by mind_initialize
     P.part = h->upload(part);
     P.det_off = h->upload(det_off);
     P.det_node = h->upload(det_node);
@@ -1726,6 +1722,7 @@ int mind_initialize(MindHandle *h) {
     CUDA_TRY(h, cudaMemsetAsync(P.inbox_count, 0, std::max(1, h->ncells) * sizeof(int32_t), h->stream));
     CUDA_TRY(h, cudaMemsetAsync(P.inbox_fill, 0, std::max(1, h->ncells) * sizeof(int32_t), h->stream));
     CUDA_TRY(h, cudaMemsetAsync(P.win_spike_count, 0, sizeof(int32_t), h->stream));
+    CUDA_TRY(h, cudaMemsetAsync(P.divide, 0, std::max(1, h->ncells), h->stream));
     int status = upload_group_state(h);
     if (status) return status;
     for (int32_t g = 0; g < P.ngroups; ++g) {
