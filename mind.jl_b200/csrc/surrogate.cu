@@ -399,7 +399,6 @@ int reserve(MindMlp *m, int64_t rows) {
     }
     MLP_CUDA(m, cudaMalloc(&m->x, cap * m->ld0 * sizeof(__nv_bfloat16)));
     MLP_CUDA(m, cudaMalloc(&m->xin, cap * m->dims[0] * sizeof(float)));
-    m->uploader.reserve(cap * m->dims[0] * sizeof(float));
     MLP_CUDA(m, cudaMalloc(&m->xt, (int64_t)m->ld0 * capT * sizeof(__nv_bfloat16)));
     MLP_CUDA(m, cudaMalloc(&m->ht_last, H * capT * sizeof(__nv_bfloat16)));
     for (int k = 0; k < 2; ++k) {
@@ -759,10 +758,6 @@ int mind_mlp_set_data(MindMlp *m, const float *x, const float *y, int64_t n) {
         cudaFree(m->data_y);
         m->data_x = m->data_y = nullptr;
         MLP_CUDA(m, cudaMalloc(&m->data_x, n * m->dims[0] * sizeof(float)));
-        // a set is usually copied once: making the buffers (about 2 ms) is repaid from 64 MB on; where
-        // predict made them, smaller sets use them too
-        const size_t bytes = n * m->dims[0] * sizeof(float);
-        if (bytes >= ((size_t)64 << 20)) m->uploader.reserve(bytes);
         MLP_CUDA(m, cudaMalloc(&m->data_y, n * sizeof(float)));
         m->data_cap = n;
     }

@@ -6,8 +6,11 @@
  * pinned buffers of its own, so that their copies to the buffers run side by side and
  * the DMA engine is always fed: 20,000 rows of 645 inputs (51.6 MB) are predicted in 2.2 ms in
  * place of 4.4, 100,000 in 10.2 in place of 23.5.  At 5 MB both take 0.43 ms, which is where the line
- * between them lies.  Like a pageable cudaMemcpyAsync, the call returns when the
- * source has been read, and the data is there for what follows on the stream.
+ * between them lies.  Making the pinned buffers takes 2-4 ms, which a network that is used
+ * once would lose: they are made by the copy with which the large ones so far come to 256 MB, where
+ * even a host whose plain copies are fast (51.6 MB in 2.9 ms a call in place of 2.2) has it back.
+ * Like a pageable cudaMemcpyAsync, the call returns when the source has been read, and the data is
+ * there for what follows on the stream.
  */
 #pragma once
 
@@ -23,6 +26,7 @@ class Uploader {
     static constexpr size_t kPiece = 512 * 1024;
     static constexpr int kThreads = 4;
     static constexpr size_t kStagedBytes = 8 * kPiece;   // smaller arrays go as they are
+    static constexpr size_t kRepaidBytes = (size_t)256 << 20;   // buffers are made for this much
 
     Uploader() = default;
     Uploader(const Uploader &) = delete;
@@ -30,7 +34,7 @@ class Uploader {
 
     /* dst (device) = src (host), `bytes` of it, on `stream`; one call at a time per object. */
     cudaError_t copy(void *dst, const void *src, size_t bytes, cudaStream_t stream) {
-        if (bytes < kStagedBytes || !staging_ || !pageable(src))
+        if (bytes < kStagedBytes || !pageable(src) || !buffers(bytes))
             return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, stream);
         int device = 0;
         cudaError_t e = cudaGetDevice(&device);
@@ -64,21 +68,6 @@ class Uploader {
         return static_cast<cudaError_t>(failed.load());
     }
 
-    /* The pinned buffers, 4 MB, for copies of `bytes` and more; where the device array grows, so that
-     * a copy allocates nothing.  Without them a copy goes as it is. */
-    void reserve(size_t bytes) {
-        if (bytes < kStagedBytes || staging_) return;
-        void *p = nullptr;
-        bool made = cudaHostAlloc(&p, 2 * kThreads * kPiece, cudaHostAllocDefault) == cudaSuccess;
-        staging_ = made ? static_cast<char *>(p) : nullptr;
-        for (cudaEvent_t &e : read_)
-            if (made) made = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
-        if (!made) {
-            (void)cudaGetLastError();
-            release();
-        }
-    }
-
     /* Gives the pinned buffers back; the streams that were copied on have been waited for. */
     void release() {
         for (cudaEvent_t &e : read_) {
@@ -87,6 +76,7 @@ class Uploader {
         }
         if (staging_) cudaFreeHost(staging_);
         staging_ = nullptr;
+        seen_ = 0;
     }
 
   private:
@@ -100,6 +90,25 @@ class Uploader {
         return a.type == cudaMemoryTypeUnregistered;
     }
 
+    /* Whether there are pinned buffers (4 MB) for a copy of `bytes`; makes them when it is time.  Where
+     * they cannot be had, copies go as they are for as much again. */
+    bool buffers(size_t bytes) {
+        if (staging_) return true;
+        seen_ = bytes < kRepaidBytes - seen_ ? seen_ + bytes : kRepaidBytes;
+        if (seen_ < kRepaidBytes) return false;
+        void *p = nullptr;
+        bool made = cudaHostAlloc(&p, 2 * kThreads * kPiece, cudaHostAllocDefault) == cudaSuccess;
+        staging_ = made ? static_cast<char *>(p) : nullptr;
+        for (cudaEvent_t &e : read_)
+            if (made) made = cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+        if (!made) {
+            (void)cudaGetLastError();
+            release();
+        }
+        return made;
+    }
+
+    size_t seen_ = 0;   // large copies so far, until the buffers are made
     char *staging_ = nullptr;
     cudaEvent_t read_[2 * kThreads] = {};
 };
