@@ -468,15 +468,25 @@ int forward(MindMlp *m, int64_t rows, bool train, cudaStream_t s, float *prob = 
     return MIND_OK;
 }
 
-/* m->xt = m->x^T on side[1], after what `s` holds so far; nothing but the first map's weight
- * gradient reads it. */
-int transpose_inputs(MindMlp *m, int64_t rows, cudaStream_t s) {
-    MLP_CUDA(m, cudaEventRecord(m->x_ready, s));
-    MLP_CUDA(m, cudaStreamWaitEvent(m->side[1], m->x_ready, 0));
+/* m->xt = m->x^T, with `beside` on side[1], after what `s` holds so far; nothing but the first map's
+ * weight gradient reads it. */
+int transpose_inputs(MindMlp *m, int64_t rows, cudaStream_t s, bool beside) {
+    cudaStream_t to = beside ? m->side[1] : s;
+    if (beside) {
+        MLP_CUDA(m, cudaEventRecord(m->x_ready, s));
+        MLP_CUDA(m, cudaStreamWaitEvent(to, m->x_ready, 0));
+    }
     const dim3 g((unsigned)((rows + 31) / 32), (unsigned)((m->ld0 + 31) / 32));
-    transpose_kernel<<<g, dim3(32, 8), 0, m->side[1]>>>(m->x, rows, m->ld0, m->ld0, m->xt, m->capT);
+    transpose_kernel<<<g, dim3(32, 8), 0, to>>>(m->x, rows, m->ld0, m->ld0, m->xt, m->capT);
     return MIND_OK;
 }
+
+/* Steps of a training call from which its captured step has the side streams of backward().  They
+ * save 12-17 us a step, but the graph with branches takes 0.35-0.7 ms more to make and to start (ms a
+ * call of 645 -> 256 x 3 -> 1 at 4,096 rows, one stream / side streams: 5 steps 0.94 / 1.23, 24 steps
+ * 3.01 / 3.08, 32 steps 3.88 / 3.85, 60 steps 6.91 / 6.54; the lines cross at 20-32 steps for batches
+ * of 64 to 16,384 rows and 3 or 6 hidden maps, and one hidden map is the same either way). */
+constexpr int32_t kBesideSteps = 32;
 
 /* Gradients of the mean loss into m->grad after transpose_inputs() and forward(train).
  *
@@ -485,17 +495,20 @@ int transpose_inputs(MindMlp *m, int64_t rows, cudaStream_t s) {
  * products depend on one another; they stay on `s`, the weight gradients (which share m->part)
  * follow one another on side[0] and the sums over rows on side[1].  dz_{l-1} overwrites the
  * buffers of dz_{l+1}, so its product waits for their readers; `s` waits for both sides at
- * the end.  Each kernel does what it did on one stream: results are bit-identical.  A training
+ * the end.  Each kernel does what it does on one stream (not `beside`): results are bit-identical.  A training
  * step of 645 -> 256 x 3 -> 1: 126.1 -> 113.6 us at 4,096 rows, 95.6 -> 78.7 at 256. */
-int backward(MindMlp *m, int64_t rows, cudaStream_t s) {
+int backward(MindMlp *m, int64_t rows, cudaStream_t s, bool beside) {
     const int32_t R = (int32_t)rows, H = m->hidden, last = m->maps - 2;
     const int64_t T = m->capT;
-    cudaStream_t wgrad = m->side[0], sums = m->side[1];
+    cudaStream_t wgrad = beside ? m->side[0] : s, sums = beside ? m->side[1] : s;
+    // one stream's order needs no events
+    auto mark = [&](cudaEvent_t e, cudaStream_t from) { return beside ? cudaEventRecord(e, from) : cudaSuccess; };
+    auto after = [&](cudaStream_t to, cudaEvent_t e) { return beside ? cudaStreamWaitEvent(to, e, 0) : cudaSuccess; };
     int cur = 0;
     for (int32_t l = last; l >= 0; --l) {
-        MLP_CUDA(m, cudaEventRecord(m->dz_ready, s));
-        MLP_CUDA(m, cudaStreamWaitEvent(wgrad, m->dz_ready, 0));
-        MLP_CUDA(m, cudaStreamWaitEvent(sums, m->dz_ready, 0));
+        MLP_CUDA(m, mark(m->dz_ready, s));
+        MLP_CUDA(m, after(wgrad, m->dz_ready));
+        MLP_CUDA(m, after(sums, m->dz_ready));
         if (l > 0) {
             // dz_{l-1} = (dz_l W_l) * SiLU'(z_{l-1}): A = dz_l rows [R x H], B = W_l^T [H x H]
             mlp::EpiParams B{};
@@ -506,8 +519,8 @@ int backward(MindMlp *m, int64_t rows, cudaStream_t s) {
             B.cols = m->dzc[cur ^ 1];
             const __nv_bfloat16 *Wt = m->wt + (int64_t)(l - 1) * H * H;
             if (l < last) {
-                MLP_CUDA(m, cudaStreamWaitEvent(s, m->wgrad_done[cur ^ 1], 0));
-                MLP_CUDA(m, cudaStreamWaitEvent(s, m->sums_done[cur ^ 1], 0));
+                MLP_CUDA(m, after(s, m->wgrad_done[cur ^ 1]));
+                MLP_CUDA(m, after(s, m->sums_done[cur ^ 1]));
             }
             MLP_TRY((product<mlp::EPI_BACK, 64>(m, m->dzr[cur], H, Wt, H, R, H, H, 1, B, s)));
         }
@@ -519,8 +532,8 @@ int backward(MindMlp *m, int64_t rows, cudaStream_t s) {
                                                     m->loss);
         }
         // side[1] also made m->xt
-        MLP_CUDA(m, cudaEventRecord(m->sums_done[cur], sums));
-        if (l == 0) MLP_CUDA(m, cudaStreamWaitEvent(wgrad, m->sums_done[cur], 0));
+        MLP_CUDA(m, mark(m->sums_done[cur], sums));
+        if (l == 0) MLP_CUDA(m, after(wgrad, m->sums_done[cur]));
         const int32_t in = l == 0 ? m->dims[0] : H;
         // dW_l^T [in x H] = h_l^T dz_l: A = h_l transposed [in x R], B = dz_l transposed [H x R];
         // stored column-major, which is dW_l [H x in] row-major, the parameters' layout
@@ -534,10 +547,10 @@ int backward(MindMlp *m, int64_t rows, cudaStream_t s) {
         MLP_TRY((product<mlp::EPI_F32, 64>(m, At, T, m->dzc[cur], T, in, H, R, splits, E, wgrad, &used)));
         split_sum_kernel<<<grid((int64_t)H * in), kT, 0, wgrad>>>(m->part, used, (int64_t)H * in,
                                                                   m->grad + m->w_off[l]);
-        MLP_CUDA(m, cudaEventRecord(m->wgrad_done[cur], wgrad));
+        MLP_CUDA(m, mark(m->wgrad_done[cur], wgrad));
         if (l == 0) {
-            MLP_CUDA(m, cudaStreamWaitEvent(s, m->wgrad_done[cur], 0));
-            MLP_CUDA(m, cudaStreamWaitEvent(s, m->sums_done[cur], 0));
+            MLP_CUDA(m, after(s, m->wgrad_done[cur]));
+            MLP_CUDA(m, after(s, m->sums_done[cur]));
         }
         cur ^= 1;
     }
@@ -738,9 +751,9 @@ int mind_mlp_gradients(MindMlp *m, const float *x, const float *y, int64_t n, fl
     MLP_TRY(reserve(m, n));
     MLP_CUDA(m, cudaMemcpyAsync(m->y, y, n * sizeof(float), cudaMemcpyHostToDevice, m->stream));
     MLP_TRY(upload_rows(m, x, n));
-    int status = transpose_inputs(m, n, m->stream);
+    int status = transpose_inputs(m, n, m->stream, true);
     if (!status) status = forward(m, n, true, m->stream);
-    if (!status) status = backward(m, n, m->stream);
+    if (!status) status = backward(m, n, m->stream, true);
     if (status) {   // nothing stays in flight on a side stream
         for (cudaStream_t s : m->side) cudaStreamSynchronize(s);
         return status;
@@ -784,14 +797,15 @@ int mind_mlp_train(MindMlp *m, int32_t steps, int32_t batch, float lr, float *lo
     const uint64_t first = (uint64_t)m->adam_t;
     MLP_CUDA(m, cudaMemcpyAsync(m->step_dev, &first, sizeof first, cudaMemcpyHostToDevice, m->stream));
     MLP_CUDA(m, cudaStreamSynchronize(m->stream));
+    const bool beside = steps >= kBesideSteps;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     MLP_CUDA(m, cudaStreamBeginCapture(m->stream, cudaStreamCaptureModeThreadLocal));
     gather_kernel<<<row_grid(batch, m->ld0), kT, 0, m->stream>>>(m->data_x, m->data_y, m->x, m->y, m->data_n,
                                                                     m->dims[0], m->ld0, batch, m->step_dev);
-    int status = transpose_inputs(m, batch, m->stream);
+    int status = transpose_inputs(m, batch, m->stream, beside);
     if (!status) status = forward(m, batch, true, m->stream);
-    if (!status) status = backward(m, batch, m->stream);
+    if (!status) status = backward(m, batch, m->stream, beside);
     adam_kernel<<<grid(m->n_params), kT, 0, m->stream>>>(m->master, m->grad, m->m1, m->m2, m->n_params, lr,
                                                          m->step_dev, C);
     step_end_kernel<<<1, 1, 0, m->stream>>>(m->step_dev, m->loss, m->loss_hist, first);
