@@ -233,19 +233,26 @@ int mind_inject_spikes(MindHandle *h, int64_t n, const int64_t *sources, const d
 /*
  * mind_autotune: the launch shape of each cell-size bin.  A bin's cells run one per CTA of
  * 128 threads (kCellThreads), 64 threads or one warp of 32 (each thread serving 1, 2 or 4
- * owner slots, so the arithmetic and its order are the same); smaller CTAs let more cells
- * share an SM (by registers and shared memory) at the price of longer parallel phases.  The
- * 128-thread launch comes compiled for two register budgets: the default, and a tight one
- * that lets 7 CTAs share an SM, which a bin starts with when its shared memory allows more
- * than 5 (the tight variant spills a few registers to L1).  The
+ * owner slots), or of 256 (two threads to an owner slot), so the arithmetic and its order are
+ * the same; smaller CTAs let more cells share an SM (by registers and shared memory) at the
+ * price of longer parallel phases.  The 128-thread launch comes compiled for two register
+ * budgets: the default, and a tight one that lets 7 CTAs share an SM, which a bin starts with
+ * when its shared memory allows more than 5 (the tight variant spills a few registers to L1).
+ * A bin starts at 128, and as long as nothing else was set or tuned it launches 256 threads
+ * where at most two detailed cells fall on an SM and a cell has more than 128 nodes (not with
+ * mechanisms compiled at run time).  The
  * call times `windows` device windows (0: 4) from a fresh initialize for the current shapes
- * and, bin by bin, for the other shapes, keeps a change that is more than 2% faster, and
+ * and, bin by bin, for 128 (exactly, at either budget), 64 and 32 threads, keeps a change that
+ * is more than 2% faster, and
  * initializes again: the state returns to t = 0 and events injected before the call are
  * dropped, as at any mind_initialize.  It needs a handle initialized at step 0 and takes the
  * precision set for it.  No reference counterpart (the reference launches fixed shapes).
- * mind_bin_threads reports the shapes (*n_bins receives the bin count), mind_set_bin_threads
- * sets them (128, 64 or 32 per bin; at least one thread per threshold detector of a cell;
- * a bin set to 128 takes the register budget it starts with).
+ * mind_bin_threads reports the shapes (*n_bins receives the bin count): 128 for a bin at its
+ * default, launched as 256 or not, else what was set or tuned.  mind_set_bin_threads
+ * sets them (256, 128, 64 or 32 per bin, which then run as given; at least one thread per
+ * threshold detector of a cell; a bin set to 128 takes the register budget it starts with;
+ * models with emitted mechanisms take 256 or 128, those with mechanisms compiled at run time
+ * and bins whose image is in HBM 128).
  */
 int mind_autotune(MindHandle *h, int32_t windows);
 int mind_bin_threads(const MindHandle *h, int32_t *threads, int32_t cap, int32_t *n_bins);

@@ -171,8 +171,9 @@ struct MindHandle {
     struct Bin {
         int32_t first, count;
         size_t smem_bytes;
-        int32_t threads = kCellThreads;   // launch shape: kCellThreads, half or a quarter
-        bool tight = false;               // 128 threads, compiled for kTightBlocks CTAs per SM
+        int32_t threads = kCellThreads;   // launch shape: kCellThreads, twice, half or a quarter
+        bool tight = false;               // at 128 threads: compiled for kTightBlocks CTAs per SM
+        bool asked = false;               // threads were set or tuned; else launch_threads may take 256 for 128
         int32_t max_detectors = 0;        // most threshold detectors on one of its cells
         int32_t max_nodes = 0;            // most nodes of one of its cells
         bool global_image = false;        // cells too large for shared memory: image in HBM
@@ -414,8 +415,7 @@ int launch_grid(int64_t work) {
     return (int)blocks;
 }
 
-/* The window kernel's launch shapes: 128 threads per cell (kCellThreads), 64, or one warp;
- * 256 where the 128-thread shape has room (`twice` in launch_window);
+/* The window kernel's launch shapes: 256 threads per cell, 128 (kCellThreads), 64, or one warp;
  * the 128-thread shapes also without the path schedule (PATHS false). */
 template <int NT, int MINB = default_min_blocks(NT), bool PATHS = true>
 cudaError_t set_window_smem(int bytes) {
@@ -439,7 +439,32 @@ int64_t resident_cells(size_t smem_bytes) {
 }
 
 bool valid_cell_threads(int32_t threads) {
-    return threads == kCellThreads || threads == kCellThreads / 2 || threads == kCellThreads / 4;
+    return threads == 2 * kCellThreads || threads == kCellThreads || threads == kCellThreads / 2 ||
+           threads == kCellThreads / 4;
+}
+
+/* Why a bin cannot run its cells with that many threads, or null. */
+const char *shape_refusal(const MindHandle *h, const MindHandle::Bin &bin, int32_t threads) {
+    if (!valid_cell_threads(threads)) return "a bin runs 256, 128, 64 or 32 threads per cell";
+    if (threads < bin.max_detectors) return "a bin's cells have more detectors than its CTA has threads";
+    if ((bin.global_image || h->gen_runtime) && threads != kCellThreads)
+        return "cells with their image in HBM, and models with mechanisms compiled at run time, run 128 threads";
+    if (h->has_generated && threads < kCellThreads) return "models with emitted mechanisms run 256 or 128 threads";
+    return nullptr;
+}
+
+/*
+ * Threads per cell of a bin's next launch: what was set, or by default 128, and 256 where there is
+ * room for them: at most two cells per multiprocessor (detailed ones; a surrogate's cells only sum
+ * their events) and more nodes than 128 threads take in one go.  The sweeps are as long, most of the
+ * rest is halved (us per step, 128 -> 256 threads: 61 trees 36.0 -> 35.1, 250 pyramidal cells
+ * 62.7 -> 58.5, 151 clamped ones 67.4 -> 62.2, 20 detailed among 1,000 surrogate cells 20.7 -> 19.3).
+ * Networks of more cells fill their registers with cells instead.
+ */
+int32_t launch_threads(const MindHandle *h, const MindHandle::Bin &bin) {
+    const bool roomy = bin.max_nodes > kCellThreads && h->ncells - h->n_sur <= 2 * 148;
+    if (bin.asked || bin.threads != kCellThreads || !roomy) return bin.threads;
+    return shape_refusal(h, bin, 2 * kCellThreads) ? bin.threads : 2 * kCellThreads;
 }
 
 int create(const MindLayout *L, MindHandle *h) {
@@ -1364,13 +1389,7 @@ void launch_window(const MindHandle *h, const MindHandle::Bin &bin, cudaStream_t
                    const int32_t *cells, int64_t n0, int32_t W) {
     constexpr int T = kCellThreads;
     const size_t smem = bin.smem_bytes;
-    // The 128-thread shape takes 256 threads per cell where there is room for it: at most two cells
-    // per multiprocessor (detailed ones; a surrogate's cells only sum their events), more nodes
-    // than 128 threads take in one go.  The sweeps are as long, most of the rest is halved (us per
-    // step, 128 -> 256 threads: 61 trees 36.0 -> 35.1, 250 pyramidal cells 62.7 -> 58.5, 151 clamped
-    // ones 67.4 -> 62.2, 20 detailed among 1,000 surrogate cells 20.7 -> 19.3).  Networks of
-    // more cells fill their registers with cells instead.
-    const bool twice = bin.threads == T && !bin.global_image && bin.max_nodes > T && h->ncells - h->n_sur <= 2 * 148;
+    const bool twice = launch_threads(h, bin) == 2 * T;
     if (h->gen_runtime) {   // the same kernel from a module compiled at run time
         const void *k = (const void *)h->rt_window[MIXED ? 1 : 0][bin.global_image ? 1 : 0];
         void *args[] = {(void *)&P, (void *)&cells, (void *)&n0, (void *)&W};
@@ -2194,26 +2213,36 @@ int mind_autotune(MindHandle *h, int32_t windows) {
     const std::pair<int32_t, bool> shapes[4] = {
         {kCellThreads, false}, {kCellThreads, true}, {kCellThreads / 2, false}, {kCellThreads / 4, false}};
     for (auto &bin : h->bins) {
-        if (bin.global_image || h->has_generated) continue;   // HBM images and emitted mechanisms: one shape
-        const std::pair<int32_t, bool> keep{bin.threads, bin.tight};
+        // the second register bound is compiled for 128 threads in shared memory, without emitted mechanisms
+        const bool bounds = !bin.global_image && !h->has_generated;
+        // the launch that a shape stands for: 128 may be 256 unless asked for, and has the two bounds
+        auto launch = [&]() {
+            const int32_t threads = launch_threads(h, bin);
+            return std::pair<int32_t, bool>{threads, bin.tight && bounds && threads == kCellThreads};
+        };
+        const MindHandle::Bin keep = bin;
+        const bool twice = launch().first > kCellThreads && !bin.asked;
         for (const auto &shape : shapes) {
-            if (shape == keep || shape.first < bin.max_detectors) continue;   // one detector per thread
-            const std::pair<int32_t, bool> before{bin.threads, bin.tight};
+            if (shape_refusal(h, bin, shape.first) || (shape.second && !bounds)) continue;
+            const MindHandle::Bin before = bin;
+            const std::pair<int32_t, bool> running = launch();
             bin.threads = shape.first;
             bin.tight = shape.second;
+            bin.asked = keep.asked || twice || shape.first != kCellThreads;
+            if (launch() == running) {
+                bin = before;
+                continue;
+            }
             double ms = 0.0;
             status = trial_ms(h, windows, &ms);
             if (status) {
-                bin.threads = keep.first;
-                bin.tight = keep.second;
+                bin = keep;
                 return status;
             }
-            if (ms < 0.98 * best) {
+            if (ms < 0.98 * best)
                 best = ms;
-            } else {
-                bin.threads = before.first;
-                bin.tight = before.second;
-            }
+            else
+                bin = before;
         }
     }
     return mind_initialize(h);
@@ -2229,16 +2258,13 @@ int mind_bin_threads(const MindHandle *h, int32_t *threads, int32_t cap, int32_t
 int mind_set_bin_threads(MindHandle *h, const int32_t *threads, int32_t n_bins) {
     if (!h || !threads || n_bins != (int32_t)h->bins.size()) return MIND_EARG;
     for (int32_t b = 0; b < n_bins; ++b) {
-        if (!valid_cell_threads(threads[b]))
-            return fail(h, MIND_EARG, "a bin runs 128, 64 or 32 threads per cell");
-        if (threads[b] < h->bins[b].max_detectors)
-            return fail(h, MIND_EARG, "a bin's cells have more detectors than its CTA has threads");
-        if ((h->bins[b].global_image || h->has_generated) && threads[b] != kCellThreads)
-            return fail(h, MIND_EARG, "cells with their image in HBM, and models with emitted mechanisms, run 128 threads");
+        const char *why = shape_refusal(h, h->bins[b], threads[b]);
+        if (why) return fail(h, MIND_EARG, why);
     }
     for (int32_t b = 0; b < n_bins; ++b) {
         MindHandle::Bin &bin = h->bins[b];
         bin.threads = threads[b];
+        bin.asked = true;
         bin.tight = threads[b] == kCellThreads && !bin.global_image && tight_by_default(bin.smem_bytes);
     }
     return MIND_OK;
