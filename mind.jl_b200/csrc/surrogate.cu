@@ -770,6 +770,7 @@ int mind_mlp_set_data(MindMlp *m, const float *x, const float *y, int64_t n) {
         cudaFree(m->data_x);
         cudaFree(m->data_y);
         m->data_x = m->data_y = nullptr;
+        m->data_n = m->data_cap = 0;   // should an allocation fail, there is no set to train from
         MLP_CUDA(m, cudaMalloc(&m->data_x, n * m->dims[0] * sizeof(float)));
         MLP_CUDA(m, cudaMalloc(&m->data_y, n * sizeof(float)));
         m->data_cap = n;
@@ -787,6 +788,7 @@ int mind_mlp_train(MindMlp *m, int32_t steps, int32_t batch, float lr, float *lo
     if (steps > m->loss_cap) {
         cudaFree(m->loss_hist);
         m->loss_hist = nullptr;
+        m->loss_cap = 0;
         MLP_CUDA(m, cudaMalloc(&m->loss_hist, (size_t)steps * sizeof(float)));
         m->loss_cap = steps;
     }
