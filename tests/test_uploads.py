@@ -1,6 +1,7 @@
 """Large copies from pageable memory (csrc/upload.hpp): when the pinned buffers are made, and every byte.
 
-Built with g++ against tests/uploads.cpp, which stands in for the CUDA runtime.
+Built with g++ against tests/uploads.cpp, which stands in for the CUDA runtime (bound to it before any
+runtime that the process has loaded).
 """
 import ctypes
 import os
@@ -17,7 +18,8 @@ MB = 1 << 20
 @pytest.fixture(scope="module")
 def lib(tmp_path_factory):
     out = str(tmp_path_factory.mktemp("uploads") / "uploads.so")
-    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-pthread", "-I", CSRC, "-I", "/usr/local/cuda/include",
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-pthread", "-Wl,-Bsymbolic", "-I", CSRC, "-I",
+                    "/usr/local/cuda/include",
                     "-o", out, os.path.join(HERE, "uploads.cpp")], check=True)
     lib = ctypes.CDLL(out)
     lib.uploader_new.restype = ctypes.c_void_p
